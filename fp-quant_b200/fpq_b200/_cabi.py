@@ -27,6 +27,7 @@ _SIGNATURES = {
     "fpq_last_error": [],
     "fpq_check_device": [c_int],
     "fpq_rotate_hadamard": [c_void_p, c_int, c_void_p, c_int, c_int64, c_int64, c_int, c_void_p],
+    "fpq_rotate_hadamard_masked": [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int, c_void_p],
     "fpq_rotate_dense": [c_void_p, c_int, c_void_p, c_int, c_int64, c_int64, c_int, c_void_p, c_void_p],
     "fpq_absmax": [c_void_p, c_int, c_int64, c_int64, c_int, c_void_p, c_void_p],
     "fpq_global_scale_update": [c_void_p, c_void_p, c_void_p, c_void_p],

@@ -131,16 +131,19 @@ def _unpack_mask(clip_mask: torch.Tensor) -> torch.Tensor:
     return bits.flatten(start_dim=-2).bool()
 
 
-def _unrotate(g: torch.Tensor, hadamard_matrix: torch.Tensor) -> torch.Tensor:
-    """`g.view(-1, h) @ hadamard_matrix.T` in bf16 (linear_fns.py:321-324): gradient with respect to the
-    rotated operand -> gradient with respect to the operand.  The normalised Sylvester matrix is symmetric,
-    so the butterfly kernel does it; any other matrix takes the dense product."""
+def _unrotate(g: torch.Tensor, mask: Optional[torch.Tensor], hadamard_matrix: torch.Tensor) -> torch.Tensor:
+    """`(g * _unpack_mask(mask)).view(-1, h) @ hadamard_matrix.T` in bf16 (linear_fns.py:321-324): gradient with
+    respect to the rotated operand -> gradient with respect to the operand, clipped elements without one.  The
+    normalised Sylvester matrix is symmetric, so the butterfly kernel does it, with the mask applied to its input;
+    any other matrix takes the dense product."""
     kind, group = kind_of(0, hadamard_matrix)
-    if kind == "identity":
-        return g
-    if kind == "hadamard":
-        return ops.rotate_hadamard(g.contiguous(), group, out_dtype=torch.bfloat16)
-    return ops.rotate_dense(g.contiguous(), hadamard_matrix.t().contiguous(), out_dtype=torch.bfloat16)
+    if kind == "dense":
+        if mask is not None:
+            g = g * _unpack_mask(mask).view_as(g).to(g.dtype)
+        return ops.rotate_dense(g.contiguous(), hadamard_matrix.t().contiguous(), out_dtype=torch.bfloat16)
+    if mask is not None:
+        return ops.rotate_hadamard_masked(g, mask, group if kind == "hadamard" else 0)
+    return g if kind == "identity" else ops.rotate_hadamard(g.contiguous(), group, out_dtype=torch.bfloat16)
 
 
 def _row_major_scales(scales: torch.Tensor, rows: int, sf_cols: int) -> torch.Tensor:
@@ -171,17 +174,13 @@ def _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale,
         w_t_fp8 = w_t_fp8[:, :out_features].contiguous()
         w_t_scales = ops.swizzle_scales(w_t_scales[:, : out_features // 32].contiguous())
     grad_input = ops.gemm_mxf8(g_fp8, w_t_fp8, g_row_scales, w_t_scales, (1.0 / weight_global_scale.float()).reshape(1))[:tokens]
-    if x_mask is not None:
-        grad_input = grad_input * _unpack_mask(x_mask).view_as(grad_input).to(grad_input.dtype)
-    grad_input = _unrotate(grad_input, hadamard_matrix).view(x_shape)
+    grad_input = _unrotate(grad_input, x_mask, hadamard_matrix).view(x_shape)
     grad_weight = None
     if want_weight_grad:
         x_t_fp8, x_t_scales = ops.mxfp4_transpose_mxfp8(x_q.view(torch.uint8), _row_major_scales(x_scales, tokens, in_features // 32),
                                                         swizzled=True)                       # [in, tokens_up128]
         grad_weight = ops.gemm_mxf8(g_t_fp8, x_t_fp8, g_col_scales, x_t_scales, (1.0 / act_global_scale.float()).reshape(1))
-        if w_mask is not None:
-            grad_weight = grad_weight * _unpack_mask(w_mask).view_as(grad_weight).to(grad_weight.dtype)
-        grad_weight = _unrotate(grad_weight, hadamard_matrix).view(out_features, in_features)
+        grad_weight = _unrotate(grad_weight, w_mask, hadamard_matrix).view(out_features, in_features)
     return grad_input, grad_weight
 
 
@@ -301,11 +300,7 @@ class FPQuant4x4MasterFn(Function):
                 x_q_pad, xs_pad = x_q, x_scales
             xt_q, xt_scales = backward_qt_bf16_op(x_q_pad, xs_pad, backward_hadamard_matrix, act_global_scale.float())
             grad_weight = matmul_mxf4_bf16_tn_op(gt_q, xt_q, gt_scales, xt_scales, ninth)
-        if x_mask is not None:
-            grad_input = grad_input * _unpack_mask(x_mask).view_as(grad_input).to(grad_input.dtype)
-        grad_input = _unrotate(grad_input, hadamard_matrix).view(ctx.x_shape)
-        if w_mask is not None:
-            grad_weight = grad_weight * _unpack_mask(w_mask).view_as(grad_weight).to(grad_weight.dtype)
-        grad_weight = _unrotate(grad_weight, hadamard_matrix).view(out_features, in_features)
+        grad_input = _unrotate(grad_input, x_mask, hadamard_matrix).view(ctx.x_shape)
+        grad_weight = _unrotate(grad_weight, w_mask, hadamard_matrix).view(out_features, in_features)
         grad_bias = g.sum(dim=0) if ctx.bias_present else None
         return grad_input, grad_weight, None, None, grad_bias, None, None, None

@@ -79,6 +79,19 @@ def rotate_hadamard(x: torch.Tensor, group: int, out_dtype: Optional[torch.dtype
     return out
 
 
+def rotate_hadamard_masked(x: torch.Tensor, mask: torch.Tensor, group: int) -> torch.Tensor:
+    """rotate(x .* mask) for a bf16 matrix x [rows, cols] and a packed clip mask u8 [rows, cols/8] (bit i of byte b =
+    element 8 b + i); group 0 masks without rotating."""
+    x, rows, cols = _2d(x)
+    mask = _cuda(mask, "mask").contiguous()
+    if x.dtype != torch.bfloat16 or mask.dtype != torch.uint8 or mask.numel() * 8 != x.numel():
+        raise ValueError("x must be bfloat16 and mask uint8 with one bit per element")
+    out = torch.empty_like(x)
+    with _guard(x.device):
+        C.call("fpq_rotate_hadamard_masked", x.data_ptr(), mask.data_ptr(), out.data_ptr(), rows, cols, group, _stream(x))
+    return out
+
+
 def rotate_dense(x: torch.Tensor, matrix: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     x, rows, cols = _2d(x)
     m = _cuda(matrix, "matrix").to(torch.float32).contiguous()

@@ -63,6 +63,15 @@ int fpq_rotate_hadamard(const void* x, int dtype_in, void* y, int dtype_out, int
                         int64_t cols, int group, fpq_stream_t stream);
 
 /*
+ * y = rotate(x .* mask), bf16 [rows, cols], `group` as above or 0 (no rotation): a clipping quantiser's gradient
+ * from the rotated operand back to the operand.  Replaces `grad * _unpack_mask(mask)` followed by the product
+ * with the Hadamard matrix (inference_lib/src/fp_quant/module/linear_fns.py:67-77, :321-324).  mask: bit i of
+ * byte b = element 8 b + i counts, [rows, cols / 8].  The mask is a factor 0 or 1, not a selection.
+ */
+int fpq_rotate_hadamard_masked(const void* x_bf16, const uint8_t* mask, void* y_bf16, int64_t rows,
+                               int64_t cols, int group, fpq_stream_t stream);
+
+/*
  * y = x.view(-1, g) @ matrix for an arbitrary g x g rotation (g in 16/32/64/128),
  * fp32 sequential accumulation over k.  Covers the identity / GSR / user matrices
  * that `forward_quantize` accepts (inference_lib/src/fp_quant/module/linear_fns.py:27-50,
