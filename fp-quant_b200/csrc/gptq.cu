@@ -21,7 +21,7 @@ namespace fpq {
 int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A, int64_t lda, int64_t a_rows,
                   int64_t a_x0, const void* B, int64_t ldb, int64_t b_rows, int64_t b_x0, bool symmetric, bool mirror,
                   int n_seg, int64_t seg_rows, const int* a_seg_y, const int* b_seg_y, float alpha, float beta,
-                  int32_t* error_flag, cudaStream_t stream, int tri = 0);
+                  int32_t* error_flag, cudaStream_t stream, int tri = 0, int64_t chain_rows = 0);
 }  // namespace fpq
 
 namespace fpq {

@@ -37,16 +37,10 @@ constexpr int NUM_THREADS = 192;
 constexpr int TMEM_COLS = 512;       // two 256-column accumulators
 
 // Two tile shapes.  128 x 256 on single CTAs with two accumulators in flight (the epilogue of a tile overlaps
-// the next tile's MMAs) for short K; 256 x 256 on CTA pairs (PairShape below) for long K, where what limits
-// the kernel is the operand traffic from L2.  (BIG = true describes the 256-row tiling the pair kernel walks;
-// the single-CTA kernel is only instantiated for BIG = false.)
-template <bool BIG>
+// the next tile's MMAs) for short K and few tiles; 256 x 256 on CTA pairs (PairShape below) otherwise.
 struct Shape {
-  static constexpr int TM = BIG ? 256 : 128;
-  static constexpr int HALVES = TM / 128;
-  static constexpr int A_BOXES = TM / 64;
-  static constexpr int STAGES = BIG ? 3 : 4;
-  static constexpr int NBUF = BIG ? 1 : 2;
+  static constexpr int A_BOXES = TILE / 64;
+  static constexpr int STAGES = 4;
   static constexpr int OFF_A = 0;
   static constexpr int OFF_B = OFF_A + STAGES * A_BOXES * BOX_BYTES;
   static constexpr int OFF_BAR = OFF_B + STAGES * B_BOXES * BOX_BYTES;   // full[S], empty[S], acc_full[2], acc_empty[2]
@@ -64,6 +58,7 @@ struct HessParams {
   int num_tiles;
   int n_seg;           // K segments
   int seg_stages;      // stages per segment: stage ks reads rows a_seg_y[ks / seg_stages] + (ks % seg_stages) * 64
+  int chain_stages;    // pair kernel: stages per accumulation chain in tensor memory (chains are added in registers)
   int symmetric;       // only tiles that touch the lower triangle
   int mirror;          // symmetric form: also write the transposed blocks above the diagonal
   int a_x0, b_x0;      // first column of A / B inside their matrices (added to the TMA x coordinate)
@@ -71,6 +66,7 @@ struct HessParams {
                        // column are skipped; 2: A^T is lower triangular (A[k, i] = 0 for k > i): stages beyond the
                        // tile's last row are skipped
   int a_seg_y[MAX_SEGMENTS], b_seg_y[MAX_SEGMENTS];
+  int vec8;            // every row of the output starts on a 32-byte boundary
   float alpha, beta;
   float* H;
   int* error_flag;
@@ -91,26 +87,57 @@ __device__ __forceinline__ uint64_t make_desc_mn_sw128(uint32_t smem_addr, uint3
 
 // Symmetric form, 128 x 256 tiles: row block ib (128 rows) needs the column tiles jb2 = 0 .. ib / 2 (256 columns
 // each).  Tiles are numbered row by row; rows 0 .. ib-1 hold q (q + 1) tiles for ib = 2 q and (q + 1)^2 for
-// ib = 2 q + 1.  256 x 256 tiles: the plain lower triangle of 256-blocks, ib (ib + 1) / 2 tiles before row ib.
-__host__ __device__ inline int tiles_before_row(int ib, bool big) {
-  if (big) return ib * (ib + 1) / 2;
+// ib = 2 q + 1.
+__host__ __device__ inline int tiles_before_row(int ib) {
   const int q = ib >> 1;
   return (ib & 1) ? (q + 1) * (q + 1) : q * (q + 1);
 }
 
-template <bool BIG>
 __device__ __forceinline__ void tile_coords(const HessParams& p, int tile, int& ib, int& jb2) {
   if (p.symmetric) {
-    int i = (int)((BIG ? 1.41421356f : 2.0f) * sqrtf((float)tile)) - 1;
+    int i = (int)(2.0f * sqrtf((float)tile)) - 1;
     if (i < 0) i = 0;
-    while (tiles_before_row(i + 1, BIG) <= tile) ++i;
-    while (tiles_before_row(i, BIG) > tile) --i;
+    while (tiles_before_row(i + 1) <= tile) ++i;
+    while (tiles_before_row(i) > tile) --i;
     ib = i;
-    jb2 = tile - tiles_before_row(i, BIG);
+    jb2 = tile - tiles_before_row(i);
   } else {
     ib = tile / p.num_blocks_n;
     jb2 = tile - ib * p.num_blocks_n;
   }
+}
+
+// 256 x 256 tiles of the pair kernel: bands of BAND row blocks, column by column inside a band, so that the 74
+// tiles in flight form a patch of about 8 x 9 blocks and read 17 blocks of the operands instead of up to 75 when
+// rows are walked one by one.  (For d = 14336 and 4096 tokens the operand alone fills the L2: row order re-read
+// most of it from HBM for each of the 56 block rows.)  The symmetric form keeps the blocks on and below the
+// diagonal: 1 + 2 + ... + r of them lie above block row r.
+constexpr int BAND = 8;
+__host__ __device__ inline int lower_tiles(int rows) { return rows * (rows + 1) / 2; }
+
+__host__ __device__ inline void pair_tile_coords(int num_blocks, int num_blocks_n, bool symmetric, int tile, int& ib,
+                                                 int& jb) {
+  if (!symmetric) {
+    const int b = tile / (BAND * num_blocks_n), left = num_blocks - b * BAND, rows = left < BAND ? left : BAND;
+    const int rem = tile - b * BAND * num_blocks_n;
+    jb = rem / rows;
+    ib = b * BAND + rem - jb * rows;
+    return;
+  }
+  int b = 0;
+  while ((b + 1) * BAND < num_blocks && lower_tiles((b + 1) * BAND) <= tile) ++b;
+  const int r0 = b * BAND, left = num_blocks - r0, rows = left < BAND ? left : BAND;
+  int rem = tile - lower_tiles(r0);
+  if (rem < r0 * rows) {                 // columns left of the band's diagonal blocks: all of its rows
+    jb = rem / rows;
+    ib = r0 + rem - jb * rows;
+    return;
+  }
+  rem -= r0 * rows;
+  int c = 0;                             // the triangle at its right end
+  while (rem >= rows - c) rem -= rows - c++;
+  jb = r0 + c;
+  ib = jb + rem;
 }
 
 // Stages [lo, hi) of every K segment that can contribute to tile (ib, jb2).
@@ -121,12 +148,11 @@ __device__ __forceinline__ void stage_range(const HessParams& p, int ib, int jb2
   if (p.tri == 2) hi = max(1, min(p.seg_stages, (ib + 1) * (TILE / BK)));
 }
 
-template <bool BIG>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const HessParams p) {
-  using Smem = Shape<BIG>;
-  constexpr int STAGES = Smem::STAGES, A_BOXES = Smem::A_BOXES, TM = Smem::TM, HALVES = Smem::HALVES, NBUF = Smem::NBUF;
+  using Smem = Shape;
+  constexpr int STAGES = Smem::STAGES, A_BOXES = Smem::A_BOXES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
@@ -176,7 +202,7 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       bool ok = true;
       for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x) {
         int ib, jb;
-        tile_coords<BIG>(p, tile, ib, jb);
+        tile_coords(p, tile, ib, jb);
         int lo, hi;
         stage_range(p, ib, jb, lo, hi);
         const int per_seg = hi - lo, n_st = per_seg * p.n_seg;
@@ -191,7 +217,7 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const int yb = p.b_seg_y[seg] + kk * BK;
 #pragma unroll
           for (int b = 0; b < A_BOXES; ++b)
-            tma_load_2d(a_dst + b * BOX_BYTES, &tmap_a, p.a_x0 + ib * TM + 64 * b, ya, bar_full + 8 * s);
+            tma_load_2d(a_dst + b * BOX_BYTES, &tmap_a, p.a_x0 + ib * TILE + 64 * b, ya, bar_full + 8 * s);
 #pragma unroll
           for (int b = 0; b < B_BOXES; ++b)
             tma_load_2d(b_dst + b * BOX_BYTES, &tmap_b, p.b_x0 + jb * TILE_N + 64 * b, yb, bar_full + 8 * s);
@@ -208,17 +234,16 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      const uint32_t idesc = make_idesc_bf16(TILE, TILE_N, true, true);   // per 128-row half
+      const uint32_t idesc = make_idesc_bf16(TILE, TILE_N, true, true);
       uint32_t it = 0, tile_count = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++tile_count) {
-        const uint32_t buf = NBUF == 2 ? (tile_count & 1) : 0;
-        const uint32_t acc_parity = NBUF == 2 ? ((tile_count >> 1) & 1) : (tile_count & 1);
+        const uint32_t buf = tile_count & 1, acc_parity = (tile_count >> 1) & 1;
         if (!mbar_wait_bounded(bar_acc_empty + 8 * buf, acc_parity ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t acc = tmem_base + buf * TILE_N;
         int ib, jb, lo, hi;
-        tile_coords<BIG>(p, tile, ib, jb);
+        tile_coords(p, tile, ib, jb);
         stage_range(p, ib, jb, lo, hi);
         const int n_st = (hi - lo) * p.n_seg;
         // one barrier wait, four MMAs and one commit per stage: every other instruction here is time the
@@ -229,12 +254,9 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint64_t a_desc = make_desc_mn_sw128(sbase + Smem::OFF_A + s * A_BOXES * BOX_BYTES, BOX_BYTES, 1024);
           const uint64_t b_desc = make_desc_mn_sw128(sbase + Smem::OFF_B + s * B_BOXES * BOX_BYTES, BOX_BYTES, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {  // 16 tokens per MMA = two 8-row atoms = 2048 bytes
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h)   // 128-row halves of the tile: boxes 2h, 2h+1 of A, accumulator h
-              tc_mma_f16(acc + h * TILE_N, a_desc + (uint64_t)((h * 2 * BOX_BYTES + k * 2048) >> 4),
-                         b_desc + (uint64_t)(k * (2048 >> 4)), idesc, (ks > 0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < BK / 16; ++k)    // 16 tokens per MMA = two 8-row atoms = 2048 bytes
+            tc_mma_f16(acc, a_desc + (uint64_t)(k * (2048 >> 4)), b_desc + (uint64_t)(k * (2048 >> 4)), idesc,
+                       (ks > 0 || k > 0) ? 1u : 0u);
           tc_commit(bar_empty + 8 * s);
         }
         if (ok) tc_commit(bar_acc_full + 8 * buf);
@@ -250,22 +272,19 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     bool ok = true;
     for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, ++tile_count) {
       int ib, jb;
-      tile_coords<BIG>(p, tile, ib, jb);
-      const uint32_t buf = NBUF == 2 ? (tile_count & 1) : 0;
-      const uint32_t acc_parity = NBUF == 2 ? ((tile_count >> 1) & 1) : (tile_count & 1);
+      tile_coords(p, tile, ib, jb);
+      const uint32_t buf = tile_count & 1, acc_parity = (tile_count >> 1) & 1;
       if (!mbar_wait_bounded(bar_acc_full + 8 * buf, acc_parity, abort_flag)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll 1
-      for (int hc = 0; hc < HALVES * (TILE_N / 32); ++hc) {
-        const int h = hc / (TILE_N / 32), c = hc % (TILE_N / 32);
-        const int rb = ib * HALVES + h;                      // 128-row block of this half
-        const int64_t i = (int64_t)rb * TILE + quarter * 32 + lane;
+      for (int c = 0; c < TILE_N / 32; ++c) {
+        const int64_t i = (int64_t)ib * TILE + quarter * 32 + lane;
         const int64_t j0 = (int64_t)jb * TILE_N + c * 32;
         const int jblock = (int)(j0 / TILE);                 // 128-column block of this chunk
-        if (j0 >= p.d2 || (p.symmetric && jblock > rb)) continue;   // beyond the matrix / above the diagonal
-        const bool mirror = p.mirror && jblock < rb;
+        if (j0 >= p.d2 || (p.symmetric && jblock > ib)) continue;   // beyond the matrix / above the diagonal
+        const bool mirror = p.mirror && jblock < ib;
         uint32_t r[32];
-        tc_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TILE_N + h * TILE_N + c * 32, r);
+        tc_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TILE_N + c * 32, r);
         tc_wait_ld();
         if (i < p.d1) {
           float* hrow = p.H + i * p.ldc + j0;
@@ -327,6 +346,13 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 // write of H) overlaps the next tile's MMAs.  Barriers as in the FP4 pair GEMM: "full" lives in the leader
 // and collects both producers' bytes, one multicast commit frees a stage in both CTAs, "accumulator full" is
 // committed to both, "accumulator empty" lives in the leader and collects the epilogue warps of both.
+//
+// A long K is walked in chains of `chain_stages` stages: each chain ends up in one of the two accumulators and is
+// added (rounded fp32 addition) to a running sum in the registers of the eight epilogue warps, 128 columns of one
+// row per thread, while the next chain's MMAs run.  The output is read and written once per tile.  Bound by the
+// tensor pipe, and by the power limit when it runs for long.  16384 tokens, one launch instead of one per 4096 tokens
+// with four epilogue warps and rows of tiles in order: d = 4096 197 us (1392 TFLOP/s) instead of 239, d = 14336
+// 2260 us (1490) instead of 2615; all of MR-GPTQ of a 4096 x 14336 linear over 262144 tokens 99.2 instead of 119.4 ms.
 struct PairShape {
   static constexpr int STAGES = 6;
   static constexpr int BOXES = 2;                                   // 64-wide boxes per operand and CTA
@@ -340,7 +366,22 @@ struct PairShape {
   static_assert(DYN_BYTES <= 227 * 1024, "stages exceed the shared memory of an SM");
 };
 
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+constexpr int PAIR_EPI_WARPS = 8;                                   // two per 32-row quarter: 128 columns each
+constexpr int PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;
+
+__device__ __forceinline__ void ld_global_f32x8(const float* p, float* v) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void st_global_f32x8(float* p, const float* v) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+               "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const HessParams p) {
   using L = PairShape;
@@ -369,7 +410,7 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_acc_full + 8 * b, 1);
-      mbar_init(bar_acc_empty + 8 * b, 8);   // four epilogue warps per CTA (used in the leader)
+      mbar_init(bar_acc_empty + 8 * b, 2 * PAIR_EPI_WARPS);   // the epilogue warps of both CTAs (used in the leader)
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -397,7 +438,7 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       bool ok = true;
       for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
         int ib, jb, lo, hi;
-        tile_coords<true>(p, tile, ib, jb);
+        pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
         stage_range(p, ib, jb, lo, hi);
         const int per_seg = hi - lo, n_st = per_seg * p.n_seg;
         const int xa = p.a_x0 + ib * 256 + (int)rank * 128, xb = p.b_x0 + jb * TILE_N + (int)rank * 128;
@@ -432,32 +473,35 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (rank == 0 && elect_one()) {
       const uint32_t peer_acc_full = map_to_cta(bar_acc_full, 1);
       const uint32_t idesc = make_idesc_bf16(256, TILE_N, true, true);
-      uint32_t it = 0, tile_count = 0;
+      uint32_t it = 0, chain_count = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs, ++tile_count) {
-        const uint32_t buf = tile_count & 1, acc_parity = (tile_count >> 1) & 1;
-        if (!mbar_wait_bounded_spin(bar_acc_empty + 8 * buf, acc_parity ^ 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t acc = tmem_base + buf * TILE_N;
+      for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
         int ib, jb, lo, hi;
-        tile_coords<true>(p, tile, ib, jb);
+        pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
         stage_range(p, ib, jb, lo, hi);
         const int n_st = (hi - lo) * p.n_seg;
-        for (int ks = 0; ks < n_st; ++ks, ++it) {
-          const uint32_t s = it % STAGES;
-          if (!mbar_wait_bounded_spin(bar_full + 8 * s, (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+        for (int k0 = 0; k0 < n_st && ok; k0 += p.chain_stages, ++chain_count) {
+          const int k1 = min(n_st, k0 + p.chain_stages);
+          const uint32_t buf = chain_count & 1, acc_parity = (chain_count >> 1) & 1;
+          if (!mbar_wait_bounded_spin(bar_acc_empty + 8 * buf, acc_parity ^ 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint64_t a_desc = make_desc_mn_sw128(sbase + L::OFF_A + s * BOXES * BOX_BYTES, BOX_BYTES, 1024);
-          const uint64_t b_desc = make_desc_mn_sw128(sbase + L::OFF_B + s * BOXES * BOX_BYTES, BOX_BYTES, 1024);
+          const uint32_t acc = tmem_base + buf * TILE_N;
+          for (int ks = k0; ks < k1; ++ks, ++it) {
+            const uint32_t s = it % STAGES;
+            if (!mbar_wait_bounded_spin(bar_full + 8 * s, (it / STAGES) & 1, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const uint64_t a_desc = make_desc_mn_sw128(sbase + L::OFF_A + s * BOXES * BOX_BYTES, BOX_BYTES, 1024);
+            const uint64_t b_desc = make_desc_mn_sw128(sbase + L::OFF_B + s * BOXES * BOX_BYTES, BOX_BYTES, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)   // 16 tokens per MMA = two 8-row atoms = 2048 bytes
-            tc_mma_f16_pair(acc, a_desc + (uint64_t)(k * (2048 >> 4)), b_desc + (uint64_t)(k * (2048 >> 4)), idesc,
-                            (ks > 0 || k > 0) ? 1u : 0u);
-          tc_commit_pair_multicast(bar_empty + 8 * s, 3);   // frees the stage in both CTAs
-        }
-        if (ok) {
-          tc_commit_pair(bar_acc_full + 8 * buf);
-          tc_commit_pair(peer_acc_full + 8 * buf);
+            for (int k = 0; k < BK / 16; ++k)   // 16 tokens per MMA = two 8-row atoms = 2048 bytes
+              tc_mma_f16_pair(acc, a_desc + (uint64_t)(k * (2048 >> 4)), b_desc + (uint64_t)(k * (2048 >> 4)), idesc,
+                              (ks > k0 || k > 0) ? 1u : 0u);
+            tc_commit_pair_multicast(bar_empty + 8 * s, 3);   // frees the stage in both CTAs
+          }
+          if (ok) {
+            tc_commit_pair(bar_acc_full + 8 * buf);
+            tc_commit_pair(peer_acc_full + 8 * buf);
+          }
         }
       }
       if (!ok) {
@@ -467,61 +511,79 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
   } else {
     // ------------------------------------------------------------- epilogue (both CTAs): H = beta H + alpha acc
-    const int quarter = warp & 3;
-    uint32_t tile_count = 0;
+    const int quarter = warp & 3, half = (warp - 2) >> 2;    // 32 rows (tensor memory lanes) x 128 columns
+    uint32_t chain_count = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs, ++tile_count) {
-      int ib, jb;
-      tile_coords<true>(p, tile, ib, jb);
-      const uint32_t buf = tile_count & 1, acc_parity = (tile_count >> 1) & 1;
-      if (!mbar_wait_bounded(bar_acc_full + 8 * buf, acc_parity, abort_flag)) { ok = false; break; }
-      tc_fence_after();
+    for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
+      int ib, jb, lo, hi;
+      pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
+      stage_range(p, ib, jb, lo, hi);
+      const int n_st = (hi - lo) * p.n_seg;
       const int rb = ib * 2 + (int)rank;                     // my 128-row block
+      const int jblock = jb * 2 + half;                      // my 128-column block
       const int64_t i = (int64_t)rb * TILE + quarter * 32 + lane;
-#pragma unroll 1
-      for (int c = 0; c < TILE_N / 32; ++c) {
-        const int64_t j0 = (int64_t)jb * TILE_N + c * 32;
-        const int jblock = (int)(j0 / TILE);
-        if (j0 >= p.d2 || (p.symmetric && jblock > rb)) continue;   // beyond the matrix / above the diagonal
-        const bool mirror = p.mirror && jblock < rb;
-        uint32_t r[32];
-        tc_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TILE_N + c * 32, r);
-        tc_wait_ld();
-        if (i < p.d1) {
-          float* hrow = p.H + i * p.ldc + j0;
-          if (j0 + 32 <= p.d2 && (p.ldc & 3) == 0) {
+      const int64_t jbase = (int64_t)jblock * TILE;
+      const bool active = jbase < p.d2 && !(p.symmetric && jblock > rb);   // not beyond the matrix / above the diagonal
+      float sum[TILE];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              float4 h = p.beta == 0.0f ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<float4*>(hrow)[q];
-              h.x = fmaf(p.beta, h.x, p.alpha * __uint_as_float(r[4 * q]));
-              h.y = fmaf(p.beta, h.y, p.alpha * __uint_as_float(r[4 * q + 1]));
-              h.z = fmaf(p.beta, h.z, p.alpha * __uint_as_float(r[4 * q + 2]));
-              h.w = fmaf(p.beta, h.w, p.alpha * __uint_as_float(r[4 * q + 3]));
-              reinterpret_cast<float4*>(hrow)[q] = h;
-              r[4 * q] = __float_as_uint(h.x); r[4 * q + 1] = __float_as_uint(h.y);
-              r[4 * q + 2] = __float_as_uint(h.z); r[4 * q + 3] = __float_as_uint(h.w);
+      for (int j = 0; j < TILE; ++j) sum[j] = 0.0f;
+      for (int k0 = 0; k0 < n_st && ok; k0 += p.chain_stages, ++chain_count) {
+        const uint32_t buf = chain_count & 1, acc_parity = (chain_count >> 1) & 1;
+        if (!mbar_wait_bounded(bar_acc_full + 8 * buf, acc_parity, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        if (active) {
+#pragma unroll
+          for (int c = 0; c < TILE / 32; ++c) {
+            uint32_t r[32];
+            tc_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TILE_N + half * TILE + c * 32, r);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(lead_acc_empty + 8 * buf);
+      }
+      if (!ok) break;
+      if (active && i < p.d1) {
+        const bool mirror = p.mirror && jblock < rb;
+#pragma unroll
+        for (int c = 0; c < TILE / 32; ++c) {
+          const int64_t j0 = jbase + c * 32;
+          float* hrow = p.H + i * p.ldc + j0;
+          float* v = sum + c * 32;
+          if (j0 + 32 <= p.d2 && p.vec8) {
+            // a lane owns 128 contiguous bytes of its row: 32-byte accesses touch whole sectors
+            float h[32];
+            if (p.beta != 0.0f) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) ld_global_f32x8(hrow + 8 * q, h + 8 * q);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) h[j] = 0.0f;
             }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = fmaf(p.beta, h[j], p.alpha * v[j]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) st_global_f32x8(hrow + 8 * q, v + 8 * q);
           } else {
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj) {
-              if (j0 + jj < p.d2) {
-                const float old = p.beta == 0.0f ? 0.0f : hrow[jj];
-                const float v = fmaf(p.beta, old, p.alpha * __uint_as_float(r[jj]));
-                hrow[jj] = v;
-                r[jj] = __float_as_uint(v);
+            for (int j = 0; j < 32; ++j) {
+              if (j0 + j < p.d2) {
+                v[j] = fmaf(p.beta, p.beta == 0.0f ? 0.0f : hrow[j], p.alpha * v[j]);
+                hrow[j] = v[j];
               }
             }
           }
           if (mirror) {
+            // H[j, i]: consecutive lanes hold consecutive i, so each store instruction is coalesced
 #pragma unroll
-            for (int jj = 0; jj < 32; ++jj)
-              if (j0 + jj < p.d2) p.H[(j0 + jj) * p.ldc + i] = __uint_as_float(r[jj]);
+            for (int j = 0; j < 32; ++j)
+              if (j0 + j < p.d2) p.H[(j0 + j) * p.ldc + i] = v[j];
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(lead_acc_empty + 8 * buf);
     }
     if (!ok && lane == 0) {
       *abort_flag = 1;
@@ -551,11 +613,13 @@ namespace fpq {
 // With more than one segment seg_rows must be a multiple of 64.  symmetric: only tiles that touch the
 // lower triangle are computed (d1 == d2); mirror: the blocks below the diagonal are also written
 // transposed.  tri = 1: B (as the [K, d2] matrix of one segment) is lower triangular, tri = 2: A^T (the
-// [d1, K] matrix) is lower triangular -- the stages that only multiply zeros are skipped.
+// [d1, K] matrix) is lower triangular -- the stages that only multiply zeros are skipped.  chain_rows > 0 (one
+// segment, a multiple of 64): rows per accumulation chain of the tensor core; chains are added with rounded fp32
+// additions, in one launch by the pair kernel and by one launch per chain on the output otherwise.
 int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A, int64_t lda, int64_t a_rows,
                   int64_t a_x0, const void* B, int64_t ldb, int64_t b_rows, int64_t b_x0, bool symmetric, bool mirror,
                   int n_seg, int64_t seg_rows, const int* a_seg_y, const int* b_seg_y, float alpha, float beta,
-                  int32_t* error_flag, cudaStream_t stream, int tri) {
+                  int32_t* error_flag, cudaStream_t stream, int tri, int64_t chain_rows) {
   if (n_seg < 1 || n_seg > MAX_SEGMENTS || (n_seg > 1 && seg_rows % BK != 0)) {
     set_error("bad K segmentation (%d segments of %lld rows)", n_seg, (long long)seg_rows);
     return FPQ_ERR_INVALID_ARGUMENT;
@@ -569,15 +633,28 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
   const int64_t rows256 = (d1 + 255) / 256, cols256 = (d2 + TILE_N - 1) / TILE_N;
   const int64_t big_tiles = symmetric ? rows256 * (rows256 + 1) / 2 : rows256 * cols256;
   const bool big = tri == 0 && total_stages >= 8 && big_tiles >= sm_count() / 2 && sm_count() >= 2;
+  if (!big && chain_rows > 0 && seg_rows > chain_rows) {
+    for (int64_t t0 = 0; t0 < seg_rows; t0 += chain_rows) {
+      const int64_t n = seg_rows - t0 < chain_rows ? seg_rows - t0 : chain_rows;
+      const int ya = (a_seg_y ? a_seg_y[0] : 0) + (int)t0, yb = (b_seg_y ? b_seg_y[0] : 0) + (int)t0;
+      if (int rc = gemm_atb_bf16(out, ldc, d1, d2, A, lda, a_rows, a_x0, B, ldb, b_rows, b_x0, symmetric,
+                                 mirror && t0 + n >= seg_rows, 1, n, &ya, &yb, alpha, t0 == 0 ? beta : 1.0f, error_flag,
+                                 stream, tri, 0))
+        return rc;
+    }
+    return FPQ_OK;
+  }
   const int tm = big ? 256 : TILE;
   p.num_blocks = (int)((d1 + tm - 1) / tm);
   p.num_blocks_n = (int)((d2 + TILE_N - 1) / TILE_N);
-  p.num_tiles = symmetric ? tiles_before_row(p.num_blocks, big) : p.num_blocks * p.num_blocks_n;
+  p.num_tiles = !symmetric ? p.num_blocks * p.num_blocks_n : big ? lower_tiles(p.num_blocks) : tiles_before_row(p.num_blocks);
   p.symmetric = symmetric ? 1 : 0;
   p.mirror = (symmetric && mirror) ? 1 : 0;
   p.a_x0 = (int)a_x0; p.b_x0 = (int)b_x0;
   p.seg_stages = (int)((seg_rows + BK - 1) / BK);
   p.n_seg = n_seg;
+  p.chain_stages = chain_rows > 0 ? (int)((chain_rows + BK - 1) / BK) : n_seg * p.seg_stages;
+  p.vec8 = ldc % 8 == 0 && ((uintptr_t)out & 31) == 0;
   p.tri = tri;
   for (int i = 0; i < n_seg; ++i) {
     p.a_seg_y[i] = a_seg_y ? a_seg_y[i] : 0;
@@ -591,8 +668,8 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
   int dev = 0;
   FPQ_CHECK_CUDA(cudaGetDevice(&dev));
   if (dev < 64 && !configured[dev]) {
-    FPQ_CHECK_CUDA(cudaFuncSetAttribute(hessian_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        Shape<false>::DYN_BYTES));
+    FPQ_CHECK_CUDA(cudaFuncSetAttribute(hessian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        Shape::DYN_BYTES));
     FPQ_CHECK_CUDA(cudaFuncSetAttribute(hessian_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         PairShape::DYN_BYTES));
     configured[dev] = true;
@@ -604,7 +681,7 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
     if (pairs < 1) return FPQ_OK;
     cudaLaunchConfig_t pc = {};
     pc.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-    pc.blockDim = dim3(NUM_THREADS, 1, 1);
+    pc.blockDim = dim3(PAIR_THREADS, 1, 1);
     pc.dynamicSmemBytes = PairShape::DYN_BYTES;
     pc.stream = stream;
     cudaLaunchAttribute pa[2];
@@ -625,14 +702,14 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Shape<false>::DYN_BYTES;
+  cfg.dynamicSmemBytes = Shape::DYN_BYTES;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = use_dependent_launch() ? 1 : 0;
-  FPQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hessian_kernel<false>, ta, tb, p));
+  FPQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, hessian_kernel, ta, tb, p));
   return FPQ_OK;
 }
 
@@ -651,18 +728,9 @@ extern "C" int fpq_hessian_accumulate(float* H, int64_t d, const void* xa_bf16, 
   const bool symmetric = xb_bf16 == nullptr || xb_bf16 == xa_bf16;
   // The tensor core truncates when it adds into its fp32 accumulator: measured on B200, every 1024 tokens
   // of one accumulation chain lower a (positive) diagonal entry by 2e-6 of its value, 1.4e-4 after 32768
-  // tokens.  The tokens are therefore taken 4096 at a time, each slab's product added to H with a correctly
-  // rounded fp32 addition in the epilogue: 4.5e-6 relative Frobenius error for any number of tokens.  Only
-  // the last slab writes the mirrored upper triangle.
-  constexpr int64_t SLAB = 4096;
-  const __nv_bfloat16* xa = reinterpret_cast<const __nv_bfloat16*>(xa_bf16);
-  const __nv_bfloat16* xb = symmetric ? xa : reinterpret_cast<const __nv_bfloat16*>(xb_bf16);
-  for (int64_t t0 = 0; t0 < tokens; t0 += SLAB) {
-    const int64_t n = tokens - t0 < SLAB ? tokens - t0 : SLAB;
-    const bool last = t0 + n >= tokens;
-    if (int rc = gemm_atb_bf16(H, d, d, d, xa + t0 * d, d, n, 0, xb + t0 * d, d, n, 0, symmetric, last, 1, n, nullptr,
-                               nullptr, alpha, t0 == 0 ? beta : 1.0f, error_flag, (cudaStream_t)stream, 0))
-      return rc;
-  }
-  return FPQ_OK;
+  // tokens.  The tokens are therefore taken in chains of 4096, whose sums are added with correctly rounded
+  // fp32 additions: 4.5e-6 relative Frobenius error for any number of tokens.
+  constexpr int64_t CHAIN = 4096;
+  return gemm_atb_bf16(H, d, d, d, xa_bf16, d, tokens, 0, symmetric ? xa_bf16 : xb_bf16, d, tokens, 0, symmetric, true, 1,
+                       tokens, nullptr, nullptr, alpha, beta, error_flag, (cudaStream_t)stream, 0, CHAIN);
 }

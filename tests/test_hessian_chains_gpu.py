@@ -1,0 +1,45 @@
+"""The accumulation chains and tile bands of the Hessian / A^T B kernel where they can go wrong: a chain of one token,
+ragged last chains, one to many bands, tiles beyond the matrix, an output whose rows are not 32-byte aligned."""
+import pytest
+import torch
+
+from tests import inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,d", [
+    (4097, 3080),        # pair kernel, second chain of one token, ragged edge tiles, two bands
+    (8192 + 4032, 4104), # three chains, 17 block rows: the last band is one row high, one column block of 8
+    (20000, 3072),       # five chains, one more than a whole number of bands
+    (9000, 1032),        # single-CTA kernel: one launch per chain
+])
+def test_chains_match_fp64(cuda_device, tokens, d):
+    """1e-5 relative Frobenius as for a single chain: chains are added with rounded fp32 additions (2^-24 each)."""
+    from fpq_b200 import ops
+
+    x = inputs.correlated_activations(tokens, d, seed=tokens).to(cuda_device)
+    h0 = torch.randn(d, d, device=cuda_device)
+    h0 = h0 + h0.t()
+    H = h0.clone()
+    ops.hessian_accumulate(H, x, alpha=0.5, beta=0.25)
+    ops.check_device_errors(cuda_device)
+    want = 0.25 * h0.double() + 0.5 * (x.double().t() @ x.double())
+    assert ((H.double() - want).norm() / want.norm()).item() < 1e-5
+    assert torch.equal(H, H.t())
+
+
+def test_output_rows_off_the_vector_alignment(cuda_device):
+    """d = 3724: rows of 14896 bytes, not a multiple of 32; the trailing updates run on CTA pairs (big enough) and take
+    the element-wise store.  fp32 chain: residual of U^T U H below 1e-3 for a Hessian of condition < 1e3."""
+    from fpq_b200 import ops
+
+    d = 3724
+    x = torch.randn(2 * d, d, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(3))
+    H = x.t() @ x / d
+    H.diagonal().add_(0.1)
+    U, status = ops.cholesky_inverse_upper(H)
+    ops.check_device_errors(cuda_device)
+    assert int(status) == 0
+    r = U.double().t() @ (U.double() @ H.double()) - torch.eye(d, device=cuda_device, dtype=torch.float64)
+    assert r.abs().max().item() < 1e-3
