@@ -555,6 +555,13 @@ __device__ __forceinline__ void process_chunk(const QuantParams& p, const RawChu
           divide_pairs(P + g * PG, PG, s[g]);
         }
       }
+    } else if (FMT == FMT_MXQUEST && sb[0] < 254u) {
+      // the divisor is a power of two with a normal reciprocal: one multiply rounds the same exact quotient
+      // (with the mask below: 8192 x 17408 in 67 us instead of 88)
+      const float r = __uint_as_float((254u - sb[0]) << 23);
+      const u64 R = pack2(r, r);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) P[j] = mul2(P[j], R);
     } else {
 #pragma unroll
       for (int g = 0; g < NG; ++g) divide_pairs(P + g * PG, PG, s[g]);
@@ -562,13 +569,15 @@ __device__ __forceinline__ void process_chunk(const QuantParams& p, const RawChu
 
     if (FMT == FMT_MXQUEST && p.mask != nullptr) {
       // bit i set = element i lies inside the grid's range (|x / 2^e| < 6, triton/mxfp4.py:105-110)
+      // = the sign of |x / 2^e| - 6 (a subtraction never rounds across zero; a NaN comes out positive), shifted in
+      // from the last element to the first
       uint32_t inside = 0;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
+      for (int j = 15; j >= 0; --j) {
         float a, b;
         unpack2(P[j], a, b);
-        inside |= (fabsf(a) < 6.0f ? 1u : 0u) << (2 * j);
-        inside |= (fabsf(b) < 6.0f ? 1u : 0u) << (2 * j + 1);
+        inside = __funnelshift_l(__float_as_uint(__fadd_rn(fabsf(b), -6.0f)), inside, 1);
+        inside = __funnelshift_l(__float_as_uint(__fadd_rn(fabsf(a), -6.0f)), inside, 1);
       }
       if (active) {
         if (MODE == MODE_CODES) {
