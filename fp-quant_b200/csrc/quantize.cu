@@ -849,53 +849,207 @@ int launch_silu_mul(const QuantParams& params, const void* up, cudaStream_t stre
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Quantise the TRANSPOSE of a bf16 matrix: x [t_rows, n] row-major -> MXFP4 of x^T [n, t_pad], rotated and
-// scaled along the t axis (groups of 32 consecutive rows of x), without materialising x^T.  This is what
-// the weight-gradient GEMM of the quantised backward pass needs of the upstream gradient
-// (backward_t_bf16, inference_lib/src/fp_quant/module/qutlass_ops.py:218-245 of IST-DASLab/FP-Quant).
-// A warp takes a 32 x 32 tile of x (32 rows of 64 bytes), turns it round through shared memory, and every
-// lane then owns one output chunk: 32 consecutive t of one column of x, i.e. exactly the chunk
-// process_chunk expects.  Rows of x beyond t_rows read as zero (t_pad may exceed t_rows).  The rotation must
-// stay inside a chunk: group 0, 16 or 32.
-constexpr int TQ_ROW_BYTES = 64 + 16;      // a tile row in shared memory, padded against bank conflicts
+// Quantise the TRANSPOSE of a matrix: x [t_rows, n] row-major -> MXFP4 of x^T [n, t_pad], rotated and scaled along the
+// t axis (groups of 32 consecutive rows of x), without materialising x^T.  Two sources:
+//   bf16: the upstream gradient, an operand of the weight-gradient GEMM of the quantised backward pass
+//         (backward_t_bf16, inference_lib/src/fp_quant/module/qutlass_ops.py:218-245 of IST-DASLab/FP-Quant);
+//   MXFP4: codes and scale bytes of the forward, dequantised, divided by *alpha and rounded to bf16 on the way
+//         (backward_qt_bf16, qutlass_ops.py:248-274), so that the bf16 transpose never goes through memory.
+// A warp takes a 32 x 32 tile of x, turns it round through shared memory as words of two consecutive t, and every
+// lane then owns one output chunk: 32 consecutive t of one column of x, i.e. exactly the chunk process_chunk
+// expects.  The next tile's loads fly meanwhile.  A warp walks four tiles along t before it changes columns, so that
+// the 16-byte pieces of an output row that share a sector are written close together.  Rows of x beyond t_rows read
+// as zero (t_pad may exceed t_rows).  The rotation must stay inside a chunk: group 0, 16 or 32.
+// @@FIG@@
+struct TransposeIn {
+  int64_t t_rows, n;
+  const uint8_t* scales;       // MXFP4 source: E8M0 bytes of the codes (in QuantParams::x), [t_rows, n / 32]
+  const float* alpha;
+  int scale_layout;
+};
 
-template <int GH, int FMT>
-__global__ void __launch_bounds__(256, 2) quant_transposed_kernel(const QuantParams p, int64_t t_rows, int64_t n) {
+// Column `col` of a tile: sixteen words of consecutive t pairs, 16-byte aligned.  Twenty words a column and eight more
+// every eight columns make both the word stores and the 128-bit loads below free of bank conflicts.
+__device__ __forceinline__ int tq_word(int col) { return col * 20 + 8 * (col >> 3); }
+constexpr int TQ_WORDS = 32 * 20 + 32;
+constexpr int TQ_RUN = 4;      // tiles along t that a warp takes together
+
+template <bool FP4IN> struct TransposeRaw;
+template <> struct TransposeRaw<false> { uint4 v[4]; };                          // eight columns of rows 2k, 2k+1, 2k+16, 2k+17
+template <> struct TransposeRaw<true> { uint2 c[2]; int e[2]; };                 // sixteen codes of rows 2k, 2k+1
+constexpr int TQ_DEAD = -100000;                                                  // "exponent" of a row beyond t_rows
+
+__device__ __forceinline__ void load_tile(const QuantParams& p, const TransposeIn& in, int64_t t0, int64_t j0, int lane,
+                                          TransposeRaw<false>& r) {
+  const int64_t col = j0 + (lane & 3) * 8;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int64_t row = t0 + (lane >> 2) * 2 + (q & 1) + 16 * (q >> 1);
+    r.v[q] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < in.t_rows && col < in.n)
+      r.v[q] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.x) + row * in.n + col));
+  }
+}
+__device__ __forceinline__ void load_tile(const QuantParams& p, const TransposeIn& in, int64_t t0, int64_t j0, int lane,
+                                          TransposeRaw<true>& r) {
+  const int64_t sf_cols = in.n / 32, ct = j0 / 32;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int64_t row = t0 + (lane >> 1) * 2 + h;
+    r.c[h] = make_uint2(0u, 0u);
+    r.e[h] = TQ_DEAD;
+    if (row < in.t_rows) {
+      r.c[h] = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const uint8_t*>(p.x) + (row * in.n + j0) / 2 + (lane & 1) * 8));
+      const size_t off = in.scale_layout == FPQ_SCALES_SWIZZLED
+                             ? swizzled_offset((uint32_t)row, (uint32_t)ct, (uint32_t)((sf_cols + 3) / 4))
+                             : (size_t)(row * sf_cols + ct);
+      r.e[h] = (int)__ldg(in.scales + off) - 127;
+    }
+  }
+}
+
+// bf16 of (E2M1 magnitude / alpha), magnitudes 2 i and 2 i + 1 in a word.
+struct QuotientTable {
+  uint32_t w[4];
+  float alpha;
+  bool usable;
+};
+__device__ __forceinline__ void make_quotients(const float* alpha, QuotientTable& t) {
+  t.alpha = *alpha;
+  t.usable = t.alpha > 9.5367e-7f && t.alpha < 1.048576e6f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(__fdiv_rn(e2m1_magnitude(2 * i), t.alpha),
+                                                   __fdiv_rn(e2m1_magnitude(2 * i + 1), t.alpha));
+    t.w[i] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+
+// The row's bf16 values of the eight magnitudes, low bytes and high bytes (once more with the sign; the zero stays +0).
+// fl((m 2^e) / a) = fl(m / a) 2^e while nothing leaves the normal range: e is added to the exponent fields.
+struct RowTable {
+  uint32_t lo_a, lo_b, hi_a, hi_b, nhi_a, nhi_b;
+};
+__device__ __forceinline__ void make_row_table(const QuotientTable& t, int e, RowTable& r) {
+  uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
+  if (e != TQ_DEAD) {
+    const uint32_t add = (uint32_t)(e * 0x00800080);        // both halves stay positive: no borrow between them
+    w0 = t.w[0] + (uint32_t)(e * 0x00800000);               // magnitude 0 stays 0
+    w1 = t.w[1] + add;
+    w2 = t.w[2] + add;
+    w3 = t.w[3] + add;
+  }
+  r.lo_a = __byte_perm(w0, w1, 0x6420); r.hi_a = __byte_perm(w0, w1, 0x7531);
+  r.lo_b = __byte_perm(w2, w3, 0x6420); r.hi_b = __byte_perm(w2, w3, 0x7531);
+  r.nhi_a = (r.hi_a | 0x80808080u) & 0xffffff00u;
+  r.nhi_b = r.hi_b | 0x80808080u;
+}
+// Four codes -> four bf16 values in two words.
+__device__ __forceinline__ void row_lookup(const RowTable& r, uint32_t x, uint32_t& w01, uint32_t& w23) {
+  const uint32_t sel = x & 0x7777u;
+  const uint32_t lo4 = __byte_perm(r.lo_a, r.lo_b, sel);
+  const uint32_t hi4 = __byte_perm(__byte_perm(r.hi_a, r.hi_b, sel), __byte_perm(r.nhi_a, r.nhi_b, sel),
+                                   ((x & 0x8888u) >> 1) | 0x3210u);
+  w01 = __byte_perm(lo4, hi4, 0x5140);
+  w23 = __byte_perm(lo4, hi4, 0x7362);
+}
+__device__ __forceinline__ uint32_t slow_quotient(uint32_t code, int e, float alpha) {
+  const float v = e == TQ_DEAD ? 0.0f : __fdiv_rn(scalbnf(e2m1_value(code), e), alpha);
+  const __nv_bfloat16 h = __float2bfloat16_rn(v + 0.0f);
+  return *reinterpret_cast<const uint16_t*>(&h);
+}
+
+__device__ __forceinline__ void store_tile(const TransposeRaw<false>& r, const QuotientTable&, int lane, uint32_t* tile) {
+  const int piece = lane & 3;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t a[4] = {r.v[2 * h].x, r.v[2 * h].y, r.v[2 * h].z, r.v[2 * h].w};
+    const uint32_t b[4] = {r.v[2 * h + 1].x, r.v[2 * h + 1].y, r.v[2 * h + 1].z, r.v[2 * h + 1].w};
+    uint32_t* dst = tile + tq_word(piece * 8) + (lane >> 2) + 8 * h;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dst[20 * j] = __byte_perm(a[j / 2], b[j / 2], (j & 1) ? 0x7632 : 0x5410);
+  }
+}
+__device__ __forceinline__ void store_tile(const TransposeRaw<true>& r, const QuotientTable& t, int lane, uint32_t* tile) {
+  const int half = lane & 1, k = lane >> 1;
+  const bool fast0 = r.e[0] == TQ_DEAD || (r.e[0] > -100 && r.e[0] < 100);
+  const bool fast1 = r.e[1] == TQ_DEAD || (r.e[1] > -100 && r.e[1] < 100);
+  if (t.usable && fast0 && fast1) {
+    RowTable ta, tb;
+    make_row_table(t, r.e[0], ta);
+    make_row_table(t, r.e[1], tb);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {                            // columns 16 half + 4 q ... + 3
+      const uint32_t wa = q < 2 ? r.c[0].x : r.c[0].y, wb = q < 2 ? r.c[1].x : r.c[1].y;
+      uint32_t a01, a23, b01, b23;
+      row_lookup(ta, (q & 1) ? wa >> 16 : wa, a01, a23);
+      row_lookup(tb, (q & 1) ? wb >> 16 : wb, b01, b23);
+      uint32_t* dst = tile + tq_word(16 * half + 4 * q) + k;
+      dst[0] = __byte_perm(a01, b01, 0x5410);
+      dst[20] = __byte_perm(a01, b01, 0x7632);
+      dst[40] = __byte_perm(a23, b23, 0x5410);
+      dst[60] = __byte_perm(a23, b23, 0x7632);
+    }
+  } else {
+    u64 ca = (u64)r.c[0].x | ((u64)r.c[0].y << 32), cb = (u64)r.c[1].x | ((u64)r.c[1].y << 32);
+#pragma unroll 1
+    for (int j = 0; j < 16; ++j, ca >>= 4, cb >>= 4)
+      tile[tq_word(16 * half + j) + k] = slow_quotient((uint32_t)ca & 15u, r.e[0], t.alpha) |
+                                         (slow_quotient((uint32_t)cb & 15u, r.e[1], t.alpha) << 16);
+  }
+}
+
+template <int GH, bool FP4IN>
+__global__ void __launch_bounds__(256, 3) quant_transposed_kernel(const QuantParams p, const TransposeIn in) {
   static_assert(GH == 0 || GH == 16 || GH == 32, "the rotation group must fit one 32-element chunk");
-  __shared__ __align__(16) uint8_t tiles[8][32 * TQ_ROW_BYTES];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  uint8_t* tile = tiles[wib];
+  __shared__ __align__(16) uint32_t tiles[8][TQ_WORDS];
+  const int lane = threadIdx.x & 31;
+  uint32_t* tile = tiles[threadIdx.x >> 5];
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   launch_dependents();
   grid_dependency_wait();
-  const int64_t col_tiles = (n + 31) / 32, t_tiles = p.chunks_per_row;      // tiles along x's columns / rows
+  QuotientTable quot{};
+  if (FP4IN) make_quotients(in.alpha, quot);
+  const int64_t col_tiles = (in.n + 31) / 32;
+  const int t_tiles = (int)p.chunks_per_row, runs = (t_tiles + TQ_RUN - 1) / TQ_RUN;
   float unused_max = 0.0f;
-  // tile index = t_tile * col_tiles + col_tile: neighbouring warps read neighbouring 64-byte pieces of the same rows
-  for (int64_t tix = warp; tix < col_tiles * t_tiles; tix += n_warps) {
-    const int64_t tt = tix / col_tiles, ct = tix - tt * col_tiles;
-    const int64_t t0 = tt * 32, j0 = ct * 32;
+  // run index = t_run * col_tiles + column tile: neighbouring warps read neighbouring pieces of the same rows
+  int64_t run = warp, ct = 0;
+  int tt = 0, t_end = 0;
+  auto start_run = [&]() {
+    const int64_t tr = run / col_tiles;
+    ct = run - tr * col_tiles;
+    tt = (int)tr * TQ_RUN;
+    t_end = min(tt + TQ_RUN, t_tiles);
+  };
+  const int64_t n_runs = col_tiles * runs;
+  TransposeRaw<FP4IN> raw;
+  if (run < n_runs) {
+    start_run();
+    load_tile(p, in, (int64_t)tt * 32, ct * 32, lane, raw);
+  }
+  while (run < n_runs) {
+    __syncwarp();                               // every lane has read the previous tile
+    store_tile(raw, quot, lane, tile);
+    const int64_t out_row = ct * 32 + lane;
+    const int chunk = tt;
+    if (++tt == t_end) {
+      run += n_warps;
+      if (run < n_runs) start_run();
+    }
+    if (run < n_runs) load_tile(p, in, (int64_t)tt * 32, ct * 32, lane, raw);
     __syncwarp();
+    RawChunk<true> c;
+    const uint4* src = reinterpret_cast<const uint4*>(tile + tq_word(lane));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int row = q * 8 + (lane >> 2), piece = lane & 3;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (t0 + row < t_rows && j0 + piece * 8 < n)
-        v = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.x) + (t0 + row) * n + j0 + piece * 8);
-      *reinterpret_cast<uint4*>(tile + row * TQ_ROW_BYTES + piece * 16) = v;
+      const uint4 w = src[q];
+      c.w[4 * q] = w.x; c.w[4 * q + 1] = w.y; c.w[4 * q + 2] = w.z; c.w[4 * q + 3] = w.w;
     }
-    __syncwarp();
-    RawChunk<true> raw;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t lo = *reinterpret_cast<const uint16_t*>(tile + (2 * k) * TQ_ROW_BYTES + lane * 2);
-      const uint32_t hi = *reinterpret_cast<const uint16_t*>(tile + (2 * k + 1) * TQ_ROW_BYTES + lane * 2);
-      raw.w[k] = lo | (hi << 16);
-    }
-    const int64_t out_row = j0 + lane;
-    const bool active = out_row < n;
-    process_chunk<GH, FMT, true, MODE_CODES>(p, raw, active ? out_row * p.chunks_per_row + tt : 0, active, lane, 0.0f, 0.0f,
-                                             unused_max);
+    const bool active = out_row < in.n;
+    process_chunk<GH, FPQ_FMT_MXFP4, true, MODE_CODES>(p, c, active ? out_row * p.chunks_per_row + chunk : 0, active, lane, 0.0f,
+                                                       0.0f, unused_max);
   }
   if (p.pad_rows != 0) {
     const int64_t n_words = (int64_t)p.pad_rows * p.sf_tiles_per_row_block;
@@ -907,13 +1061,13 @@ __global__ void __launch_bounds__(256, 2) quant_transposed_kernel(const QuantPar
   }
 }
 
-template <int GH>
-int launch_transposed(const QuantParams& params, int64_t t_rows, int64_t n, cudaStream_t stream) {
+template <int GH, bool FP4IN>
+int launch_transposed_one(const QuantParams& params, const TransposeIn& in, cudaStream_t stream) {
   QuantParams p = params;
   p.row_magic = (p.chunks_per_row >= 2 && p.n_chunks < (1ll << 32)) ? ~0ull / p.chunks_per_row + 1 : 0;
-  const int64_t tiles = ((n + 31) / 32) * (int64_t)p.chunks_per_row;
-  int64_t blocks = (int64_t)sm_count() * 2;          // persistent: two resident blocks of eight warps per SM
-  if (blocks > ceil_div64(tiles, 8)) blocks = ceil_div64(tiles, 8);
+  const int64_t runs = ((in.n + 31) / 32) * (int64_t)((p.chunks_per_row + TQ_RUN - 1) / TQ_RUN);
+  int64_t blocks = (int64_t)sm_count() * 3;          // persistent: three resident blocks of eight warps per SM
+  if (blocks > ceil_div64(runs, 8)) blocks = ceil_div64(runs, 8);
   if (blocks < 1) blocks = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)blocks, 1, 1);
@@ -924,8 +1078,33 @@ int launch_transposed(const QuantParams& params, int64_t t_rows, int64_t n, cuda
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = use_dependent_launch() ? 1 : 0;
-  FPQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, quant_transposed_kernel<GH, FPQ_FMT_MXFP4>, p, t_rows, n));
+  FPQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, quant_transposed_kernel<GH, FP4IN>, p, in));
   return FPQ_OK;
+}
+
+// x (bf16) or codes with `scales` and `alpha` (MXFP4): [t_rows, n] -> codes [n, t_pad/2] and scale bytes.
+template <bool FP4IN>
+int launch_transposed(const void* x, const uint8_t* scales, int in_layout, const float* alpha, int64_t t_rows, int64_t n,
+                      int64_t t_pad, int hadamard_group, uint8_t* codes, uint8_t* scale_bytes, int scale_layout,
+                      cudaStream_t stream) {
+  QuantParams p{};
+  p.x = x;
+  p.n_chunks = n * t_pad / 32;
+  p.chunks_per_row = (uint32_t)(t_pad / 32);
+  p.codes = codes;
+  p.sbytes = scale_bytes;
+  p.sf_tiles_per_row_block = (uint32_t)ceil_div64(t_pad / 32, 4);
+  p.layout = scale_layout;
+  if (scale_layout == FPQ_SCALES_SWIZZLED) {
+    p.rows = (uint32_t)n;
+    p.pad_rows = (uint32_t)(ceil_div64(n, 128) * 128 - n);
+  }
+  TransposeIn in{t_rows, n, scales, alpha, in_layout};
+  switch (hadamard_group) {
+    case 0: return launch_transposed_one<0, FP4IN>(p, in, stream);
+    case 16: return launch_transposed_one<16, FP4IN>(p, in, stream);
+    default: return launch_transposed_one<32, FP4IN>(p, in, stream);
+  }
 }
 
 template <int FMT>
@@ -1412,23 +1591,26 @@ extern "C" int fpq_quantize_transposed(const void* x_bf16, int64_t t_rows, int64
   FPQ_CHECK_ARG(((uintptr_t)x_bf16 & 15) == 0 && ((uintptr_t)codes & 15) == 0 && ((uintptr_t)scale_bytes & 15) == 0,
                 "pointers must be 16-byte aligned");
   FPQ_CHECK_ARG(n < ((int64_t)1 << 31) && t_pad < ((int64_t)1 << 31), "shape too large");
-  QuantParams p{};
-  p.x = x_bf16;
-  p.n_chunks = n * t_pad / 32;
-  p.chunks_per_row = (uint32_t)(t_pad / 32);
-  p.codes = codes;
-  p.sbytes = scale_bytes;
-  p.sf_tiles_per_row_block = (uint32_t)ceil_div64(t_pad / 32, 4);
-  p.layout = scale_layout;
-  if (scale_layout == FPQ_SCALES_SWIZZLED) {
-    p.rows = (uint32_t)n;
-    p.pad_rows = (uint32_t)(ceil_div64(n, 128) * 128 - n);
-  }
-  switch (hadamard_group) {
-    case 0: return launch_transposed<0>(p, t_rows, n, (cudaStream_t)stream);
-    case 16: return launch_transposed<16>(p, t_rows, n, (cudaStream_t)stream);
-    default: return launch_transposed<32>(p, t_rows, n, (cudaStream_t)stream);
-  }
+  return launch_transposed<false>(x_bf16, nullptr, 0, nullptr, t_rows, n, t_pad, hadamard_group, codes, scale_bytes,
+                                  scale_layout, (cudaStream_t)stream);
+}
+
+extern "C" int fpq_mxfp4_requantize_transposed(const uint8_t* codes_in, const uint8_t* scales_in, int scale_layout_in,
+                                               const float* alpha, int64_t t_rows, int64_t n, int64_t t_pad,
+                                               int hadamard_group, uint8_t* codes, uint8_t* scale_bytes, int scale_layout,
+                                               fpq_stream_t stream) {
+  FPQ_CHECK_ARG(codes_in && scales_in && alpha && codes && scale_bytes, "NULL pointer");
+  FPQ_CHECK_ARG(t_rows > 0 && n > 0 && n % 32 == 0, "n (%lld) must be a positive multiple of 32", (long long)n);
+  FPQ_CHECK_ARG(t_pad >= t_rows && t_pad % 32 == 0, "t_pad (%lld) must be a multiple of 32 not below t_rows", (long long)t_pad);
+  FPQ_CHECK_ARG(hadamard_group == 0 || hadamard_group == 16 || hadamard_group == 32,
+                "the rotation group of the transposing quantiser must be 0, 16 or 32 (got %d)", hadamard_group);
+  for (int layout : {scale_layout_in, scale_layout})
+    FPQ_CHECK_ARG(layout == FPQ_SCALES_ROWMAJOR || layout == FPQ_SCALES_SWIZZLED, "bad scale layout");
+  FPQ_CHECK_ARG(((uintptr_t)codes_in & 15) == 0 && ((uintptr_t)codes & 15) == 0 && ((uintptr_t)scale_bytes & 15) == 0,
+                "pointers must be 16-byte aligned");
+  FPQ_CHECK_ARG(n < ((int64_t)1 << 31) && t_pad < ((int64_t)1 << 31), "shape too large");
+  return launch_transposed<true>(codes_in, scales_in, scale_layout_in, alpha, t_rows, n, t_pad, hadamard_group, codes,
+                                 scale_bytes, scale_layout, (cudaStream_t)stream);
 }
 
 extern "C" int fpq_fake_quantize(const void* x, int dtype, int64_t rows, int64_t cols, int hadamard_group,

@@ -276,12 +276,12 @@ class FPQuant4x4MasterFn(Function):
             w_rm = _row_major_scales(w_scales, out_features, in_features // 32)
             x_rm = _row_major_scales(x_scales, tokens, in_features // 32)
             g_q, g_s, _ = ops.quantize(g, "mxfp4", gh, None, swizzled=True)
-            wt = ops.mxfp4_transpose_dequant(w_q.view(torch.uint8), w_rm, weight_global_scale.float())        # [in, out]
-            wt_q, wt_s, _ = ops.quantize(wt, "mxfp4", gh, None, swizzled=True)
+            wt_q, wt_s = ops.mxfp4_requantize_transposed(w_q.view(torch.uint8), w_rm, weight_global_scale.float(), gh,
+                                                         swizzled=True)                                        # [in, out]
             grad_input = ops.gemm_fp4(g_q, wt_q, g_s, wt_s, ninth, "mxfp4")
             gt_q, gt_s = ops.quantize_transposed(g, gh, pad_to=128, swizzled=True)                             # [out, tokens_up128]
-            xt = ops.mxfp4_transpose_dequant(x_q.view(torch.uint8), x_rm, act_global_scale.float(), pad_to=128)   # [in, tokens_up128]
-            xt_q, xt_s, _ = ops.quantize(xt, "mxfp4", gh, None, swizzled=True)
+            xt_q, xt_s = ops.mxfp4_requantize_transposed(x_q.view(torch.uint8), x_rm, act_global_scale.float(), gh, pad_to=128,
+                                                         swizzled=True)                                        # [in, tokens_up128]
             grad_weight = ops.gemm_fp4(gt_q, xt_q, gt_s, xt_s, ninth, "mxfp4")
         else:
             g_q, g_scales, _ = fused_quantize_mx_op(g, backward_hadamard_matrix, "abs_max", False)

@@ -432,6 +432,31 @@ def quantize_transposed(x: torch.Tensor, hadamard_group: int = 0, pad_to: int = 
     return codes, sb
 
 
+def mxfp4_requantize_transposed(codes: torch.Tensor, scales: torch.Tensor, alpha: torch.Tensor, hadamard_group: int = 0,
+                                pad_to: int = 32, swizzled: bool = False, scales_swizzled: bool = False):
+    """`quantize` of `mxfp4_transpose_dequant` in one pass: MXFP4 (codes u8 [t, n/2], E8M0 bytes [t, n/32], row-major or
+    in the swizzled layout) -> MXFP4 of its dequantised transpose / alpha: (codes u8 [n, t_pad/2], E8M0 bytes
+    [n, t_pad/32] row-major or swizzled).  Rotation groups 0, 16 and 32."""
+    codes = _cuda(codes, "codes").contiguous()
+    sc = _cuda(scales, "scales")
+    sc = (sc if sc.dtype == torch.uint8 else sc.view(torch.uint8)).contiguous()
+    t, n = codes.shape[0], codes.shape[1] * 2
+    want = padded_scale_shape(t, n // 32) if scales_swizzled else (t, n // 32)
+    if tuple(sc.shape) != want:
+        raise ValueError(f"scales must be {want} bytes, got {tuple(sc.shape)}")
+    if pad_to % 32 != 0:
+        raise ValueError("pad_to must be a multiple of 32")
+    alpha = _cuda(alpha, "alpha").to(torch.float32).reshape(1)
+    tp = -(-t // pad_to) * pad_to
+    out = torch.empty(n, tp // 2, dtype=torch.uint8, device=codes.device)
+    sb = _scale_buffer(n, tp // 32, swizzled, codes.device)
+    with _guard(codes.device):
+        C.call("fpq_mxfp4_requantize_transposed", codes.data_ptr(), sc.data_ptr(),
+               C.SCALES_SWIZZLED if scales_swizzled else C.SCALES_ROWMAJOR, alpha.data_ptr(), t, n, tp, hadamard_group,
+               out.data_ptr(), sb.data_ptr(), C.SCALES_SWIZZLED if swizzled else C.SCALES_ROWMAJOR, _stream(codes))
+    return out, sb
+
+
 # --------------------------------------------------------------------------- GPTQ core
 def gemm_fp4_push(a_codes: torch.Tensor, b_codes: torch.Tensor, a_scales_swizzled: torch.Tensor,
                   b_scales_swizzled: torch.Tensor, alpha: torch.Tensor, fmt: str, out: torch.Tensor, peer_ptrs,

@@ -274,6 +274,16 @@ int fpq_quantize_transposed(const void* x_bf16, int64_t t_rows, int64_t n, int64
                             uint8_t* codes, uint8_t* scale_bytes, int scale_layout, fpq_stream_t stream);
 
 /*
+ * The same for a matrix that is itself MXFP4 (codes [t_rows, n/2], E8M0 bytes in either layout): MXFP4 of the
+ * transpose of bf16(dequantised / *alpha).  backward_qt_bf16 (qutlass_ops.py:248-274) in one pass:
+ * fpq_mxfp4_transpose_dequant followed by fpq_quantize, bit for bit, without the bf16 matrix between them.
+ * n % 32 == 0; rotation group 0, 16 or 32.
+ */
+int fpq_mxfp4_requantize_transposed(const uint8_t* codes_in, const uint8_t* scales_in, int scale_layout_in,
+                                    const float* alpha, int64_t t_rows, int64_t n, int64_t t_pad, int hadamard_group,
+                                    uint8_t* codes, uint8_t* scale_bytes, int scale_layout, fpq_stream_t stream);
+
+/*
  * Column-parallel form of fpq_gemm_fp4 for tensor parallelism over NVLink (no counterpart in the reference,
  * which is single-GPU, README.md:92): this rank holds N of the layer's ldc output features, starting at
  * col_offset.  Its [M, N] product is written into columns [col_offset, col_offset + N) of its own
