@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(THREADS) square_quantize_kernel(const __nv_bfl
 __global__ void __launch_bounds__(THREADS) fp4_transpose_fp8_kernel(const uint8_t* __restrict__ codes,
                                                                     const uint8_t* __restrict__ scales, int64_t rows,
                                                                     int64_t cols, int64_t rows_pad, uint8_t* __restrict__ out,
-                                                                    uint8_t* __restrict__ out_scales, int layout) {
+                                                                    uint8_t* __restrict__ out_scales, int layout,
+                                                                    int layout_in) {
   __shared__ float sm[SQ_PER_BLOCK][SQ + 1];
   __shared__ __align__(16) uint8_t tile[SQ_PER_BLOCK * T8_SQ];
   const int r = threadIdx.x / SQ_PER_BLOCK, c = threadIdx.x % SQ_PER_BLOCK;
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(THREADS) fp4_transpose_fp8_kernel(const uint8_
   int e_row = -1000;                                   // below every real exponent
   if (live) {
     w = *reinterpret_cast<const uint4*>(codes + row * (cols / 2) + col0 / 2);
-    e_row = (int)scales[row * (cols / SQ) + sq_col] - 127;
+    e_row = (int)scales[sf_offset(row, sq_col, cols / SQ, layout_in)] - 127;
   }
   const int emax = (int)square_max((float)e_row, r, c, sm);
   uint32_t byte = 0;
@@ -325,6 +326,8 @@ extern "C" int fpq_quantize_mxfp8_square(const void* x_bf16, int64_t rows, int64
 extern "C" int fpq_mxfp4_transpose_mxfp8(const uint8_t* codes, const uint8_t* scales_rowmajor, int64_t rows, int64_t cols,
                                          uint8_t* out_e4m3, uint8_t* out_scales, int scale_layout, fpq_stream_t stream) {
   FPQ_CHECK_ARG(codes && scales_rowmajor && out_e4m3 && out_scales, "NULL pointer");
+  const int layout_in = scale_layout & FPQ_SCALES_INPUT_SWIZZLED ? FPQ_SCALES_SWIZZLED : FPQ_SCALES_ROWMAJOR;
+  scale_layout &= ~FPQ_SCALES_INPUT_SWIZZLED;
   FPQ_CHECK_ARG(scale_layout == FPQ_SCALES_ROWMAJOR || scale_layout == FPQ_SCALES_SWIZZLED, "bad scale layout");
   FPQ_CHECK_ARG(rows > 0 && cols > 0 && cols % 32 == 0, "cols (%lld) must be a positive multiple of 32", (long long)cols);
   FPQ_CHECK_ARG(rows < (1ll << 31) && cols < (1ll << 31), "shape too large");
@@ -333,7 +336,7 @@ extern "C" int fpq_mxfp4_transpose_mxfp8(const uint8_t* codes, const uint8_t* sc
   const dim3 grid((unsigned)((cols / SQ + SQ_PER_BLOCK - 1) / SQ_PER_BLOCK), (unsigned)(rows_pad / SQ));
   FPQ_CHECK_ARG(grid.y < 65536, "too many rows for one launch");
   fp4_transpose_fp8_kernel<<<grid, THREADS, 0, (cudaStream_t)stream>>>(codes, scales_rowmajor, rows, cols, rows_pad, out_e4m3,
-                                                                       out_scales, scale_layout);
+                                                                       out_scales, scale_layout, layout_in);
   FPQ_CHECK_LAUNCH();
   return FPQ_OK;
 }

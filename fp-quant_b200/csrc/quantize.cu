@@ -1781,3 +1781,37 @@ extern "C" int fpq_swizzle_scales(const uint8_t* rowmajor, int64_t rows, int64_t
   FPQ_CHECK_LAUNCH();
   return FPQ_OK;
 }
+
+// Rotate + quantise and the FP4 GEMM in one call: what a linear layer does per forward pass.  The activations' codes and
+// swizzled scale bytes go to the caller's workspace.  A decode step is bound by the host: two calls with their tensor
+// wrappers and checks cost more than the two kernels.
+extern "C" int64_t fpq_linear_workspace_bytes(int64_t M, int64_t K, int format) {
+  if (M < 0 || K <= 0) return 0;
+  const int g = format == FPQ_FMT_NVFP4 ? 16 : 32;
+  const int64_t codes = (M * (K / 2) + 255) & ~(int64_t)255;
+  return codes + ((M + 127) & ~(int64_t)127) * ((K / g + 3) & ~(int64_t)3);
+}
+
+extern "C" int fpq_linear_forward(const void* x_bf16, const void* up_bf16, int64_t M, int64_t N, int64_t K,
+                                  int hadamard_group, int format, int quest, const float* global_scale,
+                                  const uint8_t* w_codes, const uint8_t* w_scales_swizzled, const float* alpha,
+                                  const void* bias_bf16, void* workspace, int64_t workspace_bytes, void* out_bf16,
+                                  int32_t* error_flag, fpq_stream_t stream) {
+  FPQ_CHECK_ARG(workspace != nullptr && ((uintptr_t)workspace & 255) == 0, "the workspace must be non-NULL and 256-byte aligned");
+  FPQ_CHECK_ARG(workspace_bytes >= fpq_linear_workspace_bytes(M, K, format), "the workspace is too small");
+  FPQ_CHECK_ARG(!quest || (format == FPQ_FMT_MXFP4 && up_bf16 == nullptr), "QuEST scales are an MXFP4 rule without the fused SiLU");
+  const int g = format == FPQ_FMT_NVFP4 ? 16 : 32;
+  uint8_t* codes = reinterpret_cast<uint8_t*>(workspace);
+  uint8_t* sb = codes + ((M * (K / 2) + 255) & ~(int64_t)255);
+  if ((K / g) % 4 != 0 && M > 0)       // scale columns up to the next multiple of four: zero (pad rows: the quantise kernel)
+    FPQ_CHECK_CUDA(cudaMemsetAsync(sb, 0, (size_t)(((M + 127) & ~(int64_t)127) * ((K / g + 3) & ~(int64_t)3)), (cudaStream_t)stream));
+  int rc;
+  if (up_bf16)
+    rc = fpq_quantize_silu_mul(x_bf16, up_bf16, M, K, hadamard_group, format, global_scale, codes, sb, FPQ_SCALES_SWIZZLED, stream);
+  else if (quest)
+    rc = fpq_quantize_quest(x_bf16, FPQ_DT_BF16, M, K, hadamard_group, codes, sb, FPQ_SCALES_SWIZZLED, nullptr, stream);
+  else
+    rc = fpq_quantize(x_bf16, FPQ_DT_BF16, M, K, hadamard_group, format, global_scale, codes, sb, FPQ_SCALES_SWIZZLED, nullptr, stream);
+  if (rc != FPQ_OK) return rc;
+  return fpq_gemm_fp4(codes, w_codes, sb, w_scales_swizzled, alpha, bias_bf16, out_bf16, M, N, K, format, error_flag, stream);
+}

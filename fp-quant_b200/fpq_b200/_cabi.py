@@ -15,7 +15,7 @@ LIB_PATH = os.path.join(_HERE, "lib", "libfpq_b200.so")
 FPQ_OK = 0
 FMT_MXFP4, FMT_NVFP4 = 0, 1
 DT_BF16, DT_F32 = 0, 1
-SCALES_ROWMAJOR, SCALES_SWIZZLED = 0, 1
+SCALES_ROWMAJOR, SCALES_SWIZZLED, SCALES_INPUT_SWIZZLED = 0, 1, 16
 OUT_CODES, OUT_GRID, OUT_DEQUANT, OUT_DEQUANT_STE = 0, 1, 2, 3
 RELATIVE_MSE_ACC_DOUBLES = 32768
 ERR_DEVICE_TIMEOUT = -4
@@ -63,6 +63,9 @@ _SIGNATURES = {
     "fpq_quantize_mxfp8_square": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "fpq_mxfp4_transpose_mxfp8": [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_void_p],
     "fpq_mxfp4_transpose_dequant": [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_void_p],
+    "fpq_linear_workspace_bytes": [c_int64, c_int64, c_int],
+    "fpq_linear_forward": [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                           c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p],
     "fpq_quantize_transposed": [c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "fpq_mxfp4_requantize_transposed": [c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p,
                                         c_void_p, c_int, c_void_p],
@@ -70,7 +73,7 @@ _SIGNATURES = {
                       c_void_p, c_void_p],
 }
 _RESTYPES = {"fpq_last_error": c_char_p, "fpq_cholesky_workspace_floats": c_int64,
-             "fpq_gptq_workspace_bytes": c_int64}
+             "fpq_gptq_workspace_bytes": c_int64, "fpq_linear_workspace_bytes": c_int64}
 
 _lib = None
 

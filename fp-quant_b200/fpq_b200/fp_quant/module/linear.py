@@ -10,10 +10,10 @@ import torch
 from torch import nn
 
 from ... import ops
-from ...rotation import sylvester
+from ...rotation import classify_rotation, sylvester
 from ..utils.config import FPQuantConfig, FPQuantDtype, validate_config
 from .linear_fns import (FPQuant4x4MasterFn, FPQuant4x8MasterFn, FPQuant4x8NoMasterFn, FPQuant4x16MasterFn, FPQuant4x16NoMasterFn,
-                         _linear_forward, forward_gemm_blocked, forward_quantize, gemm_alpha)
+                         GemmConstants, _linear_forward, forward_gemm_blocked, forward_quantize, gemm_alpha, plain_eager)
 from .pseudoquant_linear_fns import PseudoQuant4x16MasterFn, PseudoQuant4x16NoMasterFn, forward_pseudoquantize
 from .qutlass_ops import (HAS_QUTLASS, fused_silu_mul_quantize_blocked_op,  # noqa: F401  (HAS_QUTLASS: API compatibility)
                           swizzle_scales_op)
@@ -63,8 +63,8 @@ class FPQuantLinear(nn.Module):
         self.register_buffer("backward_hadamard_matrix", torch.empty(hg, hg, **kw))
         self._scales_blocked = None
         self._scales_blocked_key = None
-        self._alpha = None
-        self._alpha_key = None
+        self._constants = None
+        self._constants_of = None
 
     # ------------------------------------------------------------------ load-time step
     @torch.no_grad()
@@ -125,16 +125,49 @@ class FPQuantLinear(nn.Module):
             self._scales_blocked_key = key
         return self._scales_blocked
 
-    def _gemm_alpha(self) -> torch.Tensor:
-        """1 / (weight_global_scale * act_global_scale) as fp32 [1], recomputed only when a tensor scale changed
-        (three small kernels per forward otherwise: the decode path is bound by launches)."""
+    def _gemm_constants(self) -> GemmConstants:
+        """What the passes derive from the two tensor scales, recomputed only when one of them changed (up to nine small
+        kernels per training step otherwise).  The tensors it was made from are kept and compared as objects, so an
+        address that is used again cannot pass for them."""
         w, a = self.weight_global_scale, self.act_global_scale
+        of = self._constants_of
+        if of is None or of[0] is not w or of[1] is not a or of[2:] != (w._version, a._version, w.data_ptr(), a.data_ptr()):
+            self._constants = GemmConstants.make(w, a)
+            self._constants_of = (w, a, w._version, a._version, w.data_ptr(), a.data_ptr())
+        return self._constants
+
+    def _gemm_alpha(self) -> torch.Tensor:
+        """1 / (weight_global_scale * act_global_scale) as fp32 [1]."""
         if torch.compiler.is_compiling():
-            return gemm_alpha(w, a)
-        key = (w.data_ptr(), w._version, a.data_ptr(), a._version)
-        if self._alpha is None or self._alpha_key != key:
-            self._alpha, self._alpha_key = gemm_alpha(w, a), key
-        return self._alpha
+            return gemm_alpha(self.weight_global_scale, self.act_global_scale)
+        return self._gemm_constants().alpha
+
+    def _fused_forward(self, x: torch.Tensor, up: torch.Tensor = None):
+        """Inference through pre-quantised weights as one native call, or None where that does not cover the call (a
+        tracer or a tensor subclass at work, other devices and types, a dense rotation, a bias that is not bf16): the
+        general path then takes it, or refuses it."""
+        cfg = self.config
+        wq, matrix, gs, bias = self.qweight, self.forward_hadamard_matrix, self.act_global_scale, self.bias
+        quest = cfg.forward_method == "quest"
+        nv = cfg.forward_dtype == FPQuantDtype.NVFP4
+        if (wq is None or not plain_eager(x) or not x.is_cuda or wq.device != x.device or x.dim() < 2 or x.numel() == 0
+                or x.shape[-1] != self.in_features or wq.shape[1] * 2 != self.in_features or not wq.is_contiguous()
+                or matrix.dtype != torch.bfloat16 or gs.device != x.device
+                or (bias is not None and (bias.dtype != torch.bfloat16 or bias.device != x.device or not bias.is_contiguous()))
+                or not (cfg.forward_method == "abs_max" or (quest and not nv and up is None))):
+            return None
+        kind, group = classify_rotation(matrix)
+        if kind == "dense":
+            return None
+        if x.dtype != torch.bfloat16:
+            x = x.to(torch.bfloat16)
+        if not x.is_contiguous():
+            x = x.contiguous()
+        if up is not None and not up.is_contiguous():
+            up = up.contiguous()
+        consts = self._gemm_constants()
+        return ops.linear_forward(x, up, wq, self._blocked_weight_scales(), consts.alpha, "nvfp4" if nv else "mxfp4",
+                                  group if kind == "hadamard" else 0, quest, consts.act_scale, bias)
 
     def forward_silu_mul(self, gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
         """`self(silu(gate) * up)` for the down-projection of a gated MLP, with the activation computed inside
@@ -148,6 +181,10 @@ class FPQuantLinear(nn.Module):
                  and gate.dtype == torch.bfloat16 and up.dtype == torch.bfloat16 and gate.is_cuda)
         if not fused:
             return self.forward(torch.nn.functional.silu(gate) * up)
+        if up.shape == gate.shape and up.device == gate.device and plain_eager(up):
+            y = self._fused_forward(gate, up)
+            if y is not None:
+                return y
         lead = gate.shape[:-1]
         g2, u2 = gate.contiguous().flatten(end_dim=-2), up.contiguous().flatten(end_dim=-2)
         nv = cfg.forward_dtype == FPQuantDtype.NVFP4
@@ -161,9 +198,18 @@ class FPQuantLinear(nn.Module):
             y = y + self.bias
         return y.unflatten(dim=0, sizes=lead)
 
+    def _training_constants(self, x: torch.Tensor):
+        """The cached constants for a training pass; None (they are derived on the way) under a tracer."""
+        return self._gemm_constants() if plain_eager(x) else None
+
     # ------------------------------------------------------------------ forward
     def forward(self, x) -> torch.Tensor:
         cfg = self.config
+        if not cfg.store_master_weights and not cfg.pseudoquantization and cfg.backward_dtype == FPQuantDtype.BF16 \
+                and not (torch.is_grad_enabled() and x.requires_grad):
+            y = self._fused_forward(x)
+            if y is not None:
+                return y
         fp4 = cfg.forward_dtype in (FPQuantDtype.MXFP4, FPQuantDtype.NVFP4)
         if fp4 and cfg.backward_dtype == FPQuantDtype.BF16:
             common = (self.weight_global_scale, self.act_global_scale, self.bias, self.forward_hadamard_matrix,
@@ -173,7 +219,7 @@ class FPQuantLinear(nn.Module):
                     return PseudoQuant4x16MasterFn.apply(x, self.weight, *common)
                 return PseudoQuant4x16NoMasterFn.apply(x, self.dqweight, *common)
             if cfg.store_master_weights:
-                return FPQuant4x16MasterFn.apply(x, self.weight, *common)
+                return FPQuant4x16MasterFn.apply(x, self.weight, *common, self._training_constants(x))
             if not (torch.is_grad_enabled() and x.requires_grad):
                 # inference: the function body without the autograd.Function wrapper (its backward only raises)
                 return _linear_forward(x, self.qweight, self._blocked_weight_scales(), *common, self._gemm_alpha())
@@ -183,12 +229,13 @@ class FPQuantLinear(nn.Module):
             common = (self.weight_global_scale, self.act_global_scale, self.bias, self.forward_hadamard_matrix,
                       cfg.forward_dtype, cfg.forward_method)
             if cfg.store_master_weights:
-                return FPQuant4x8MasterFn.apply(x, self.weight, *common)
+                return FPQuant4x8MasterFn.apply(x, self.weight, *common, self._training_constants(x))
             return FPQuant4x8NoMasterFn.apply(x, self.qweight, self.scales, *common)
         if cfg.forward_dtype == FPQuantDtype.MXFP4 and cfg.backward_dtype == FPQuantDtype.MXFP4 and not cfg.pseudoquantization \
                 and cfg.store_master_weights:
             return FPQuant4x4MasterFn.apply(x, self.weight, self.weight_global_scale, self.act_global_scale, self.bias,
-                                            self.forward_hadamard_matrix, cfg.forward_dtype, cfg.forward_method)
+                                            self.forward_hadamard_matrix, cfg.forward_dtype, cfg.forward_method,
+                                            self._training_constants(x))
         raise ValueError(
             f"Forward dtype: {cfg.forward_dtype}, backward dtype: {cfg.backward_dtype}, store_master_weights: "
             f"{cfg.store_master_weights}, pseudoquantization: {cfg.pseudoquantization} isn't supported yet.")

@@ -6,7 +6,7 @@ weights raises like the reference does.  `FPQuant4x4MasterFn` runs both gradient
 """
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import NamedTuple, Optional, Tuple
 
 import torch
 from torch.autograd import Function
@@ -19,6 +19,28 @@ from .qutlass_ops import (backward_bf16_square_double_mxfp8_op, backward_qt_bf16
                           fused_quantize_nv_op, matmul_fp4_bf16_tn_blocked_op, matmul_mxf4_bf16_tn_op,
                           matmul_mxf8_bf16_nn_op, matmul_mxf8_bf16_tn_op, matmul_nvf4_bf16_tn_op,
                           mxfp4_transpose_mxfp8_op)
+
+
+def plain_eager(x: torch.Tensor) -> bool:
+    """No tracer, dispatch mode, functorch transform or tensor subclass between the caller and the kernels: the native calls
+    may be made without the registered ops (85 us of dispatch each)."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None)
+
+
+class GemmConstants(NamedTuple):
+    """fp32 [1] tensors that follow from the two tensor scales."""
+    alpha: torch.Tensor          # `gemm_alpha`
+    act_scale: torch.Tensor
+    weight_scale: torch.Tensor
+    act_inverse: torch.Tensor    # 1 / act_scale
+    weight_inverse: torch.Tensor
+
+    @classmethod
+    @torch.no_grad()
+    def make(cls, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor) -> "GemmConstants":
+        w, a = weight_global_scale.float().reshape(1), act_global_scale.float().reshape(1)
+        return cls(gemm_alpha(weight_global_scale, act_global_scale), a, w, 1.0 / a, 1.0 / w)
 
 
 def forward_quantize(x: torch.Tensor, hadamard_matrix: torch.Tensor, global_scale: torch.Tensor,
@@ -106,11 +128,15 @@ class FPQuant4x16MasterFn(Function):
 
     @staticmethod
     def forward(ctx, x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype,
-                forward_method):
+                forward_method, constants: Optional[GemmConstants] = None):
+        """`constants` (optional): what follows from the two tensor scales, made once by the module."""
+        alpha = None
+        if constants is not None:
+            alpha, act_global_scale, weight_global_scale = constants.alpha, constants.act_scale, constants.weight_scale
         w_q, w_scales = forward_quantize_blocked(weight, forward_hadamard_matrix, weight_global_scale, dtype,
                                                  forward_method)
         y = _linear_forward(x, w_q, w_scales, weight_global_scale, act_global_scale, bias,
-                            forward_hadamard_matrix, dtype, forward_method)
+                            forward_hadamard_matrix, dtype, forward_method, alpha)
         ctx.x_shape, ctx.bias_present = x.shape, bias is not None
         ctx.save_for_backward(x.contiguous().flatten(end_dim=-2), weight)
         return y
@@ -122,7 +148,7 @@ class FPQuant4x16MasterFn(Function):
         grad_input = (g @ weight).view(ctx.x_shape)
         grad_weight = g.t() @ x_flat
         grad_bias = g.sum(dim=0) if ctx.bias_present else None
-        return grad_input, grad_weight, None, None, grad_bias, None, None, None
+        return grad_input, grad_weight, None, None, grad_bias, None, None, None, None
 
 
 def _unpack_mask(clip_mask: torch.Tensor) -> torch.Tensor:
@@ -152,7 +178,7 @@ def _row_major_scales(scales: torch.Tensor, rows: int, sf_cols: int) -> torch.Te
 
 
 def _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale, weight_global_scale, x_mask, w_mask,
-                    hadamard_matrix, x_shape, want_weight_grad: bool):
+                    hadamard_matrix, x_shape, want_weight_grad: bool, swizzled: bool = False, constants=None):
     """The two gradient GEMMs of linear_fns.py:270-350 on MXFP8 operands.  The saved MXFP4 operands are
     transposed into MXFP8 (exactly, unless the scales of a 32-row band differ by more than 2^14), the bf16
     gradient is quantised once with a scale per 32 x 32 square and read along either axis.
@@ -160,28 +186,75 @@ def _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale,
     Same data flow as the reference's `mxfp4_transpose_mxfp8_op` / `backward_bf16_square_double_mxfp8_op` /
     `matmul_mxf8_bf16_tn_op` / `..._nn_op` sequence, with the re-layouts folded into the producers: the
     quantisers write their scales in the layout the GEMM reads, and the gradient's bytes come out in both
-    orientations, so the `nn` product is a `tn` product of the transposed copy."""
+    orientations, so the `nn` product is a `tn` product of the transposed copy.  `swizzled`: x_scales and w_scales
+    already are in the layout the GEMM reads."""
+    if constants is not None:
+        act_inverse, weight_inverse = constants.act_inverse, constants.weight_inverse
+    else:
+        act_inverse, weight_inverse = ((1.0 / s.float()).reshape(1) for s in (act_global_scale, weight_global_scale))
+
+    def operand_scales(scales, rows):
+        return scales.view(torch.uint8) if swizzled else _row_major_scales(scales, rows, in_features // 32)
+
     g = grad_output.flatten(end_dim=-2).to(torch.bfloat16).contiguous()
     tokens, out_features = g.shape
     in_features = w_q.size(-1) * 2
     g_fp8, g_row_scales, g_col_scales, g_t_fp8 = ops.quantize_mxfp8_square(g, swizzled=True, transposed=want_weight_grad) \
         if want_weight_grad else ops.quantize_mxfp8_square(g, swizzled=True) + (None,)
     if out_features % 128 == 0:
-        w_t_fp8, w_t_scales = ops.mxfp4_transpose_mxfp8(w_q.view(torch.uint8), _row_major_scales(w_scales, out_features, in_features // 32),
-                                                        swizzled=True)
+        w_t_fp8, w_t_scales = ops.mxfp4_transpose_mxfp8(w_q.view(torch.uint8), operand_scales(w_scales, out_features), swizzled=True,
+                                                        scales_swizzled=swizzled)
     else:     # the transposed weight is padded along the contraction axis: cut it back to the gradient's width
-        w_t_fp8, w_t_scales = ops.mxfp4_transpose_mxfp8(w_q.view(torch.uint8), _row_major_scales(w_scales, out_features, in_features // 32))
+        w_t_fp8, w_t_scales = ops.mxfp4_transpose_mxfp8(w_q.view(torch.uint8), operand_scales(w_scales, out_features), scales_swizzled=swizzled)
         w_t_fp8 = w_t_fp8[:, :out_features].contiguous()
         w_t_scales = ops.swizzle_scales(w_t_scales[:, : out_features // 32].contiguous())
-    grad_input = ops.gemm_mxf8(g_fp8, w_t_fp8, g_row_scales, w_t_scales, (1.0 / weight_global_scale.float()).reshape(1))[:tokens]
+    grad_input = ops.gemm_mxf8(g_fp8, w_t_fp8, g_row_scales, w_t_scales, weight_inverse)[:tokens]
     grad_input = _unrotate(grad_input, x_mask, hadamard_matrix).view(x_shape)
     grad_weight = None
     if want_weight_grad:
-        x_t_fp8, x_t_scales = ops.mxfp4_transpose_mxfp8(x_q.view(torch.uint8), _row_major_scales(x_scales, tokens, in_features // 32),
-                                                        swizzled=True)                       # [in, tokens_up128]
-        grad_weight = ops.gemm_mxf8(g_t_fp8, x_t_fp8, g_col_scales, x_t_scales, (1.0 / act_global_scale.float()).reshape(1))
+        x_t_fp8, x_t_scales = ops.mxfp4_transpose_mxfp8(x_q.view(torch.uint8), operand_scales(x_scales, tokens), swizzled=True,
+                                                        scales_swizzled=swizzled)                       # [in, tokens_up128]
+        grad_weight = ops.gemm_mxf8(g_t_fp8, x_t_fp8, g_col_scales, x_t_scales, act_inverse)
         grad_weight = _unrotate(grad_weight, w_mask, hadamard_matrix).view(out_features, in_features)
     return grad_input, grad_weight
+
+
+def _training_forward(x, weight, weight_global_scale, act_global_scale, bias, hadamard_matrix, dtype, forward_method,
+                      constants: Optional[GemmConstants], direct: bool = True):
+    """Forward pass of the MXFP4 layers whose backward runs on quantised operands: (y, (codes, scales, clip mask) of x and
+    of the weight, whether the scales are swizzled).  Where `direct` allows it and the calls need not be traced, the
+    kernels are called directly and the scales stay in the layout that the matmul reads; otherwise the reference's op
+    sequence with its row-major scales."""
+    x_flat = x.contiguous().flatten(end_dim=-2)
+    matrix = hadamard_matrix.to(torch.bfloat16)
+    direct = (direct and constants is not None and dtype == FPQuantDtype.MXFP4 and forward_method in ("abs_max", "quest")
+              and plain_eager(x) and plain_eager(weight) and kind_of(0, matrix)[0] != "dense")
+    if direct:
+        kind, group = kind_of(0, matrix)
+        group = group if kind == "hadamard" else 0
+
+        def quantize(t):
+            t16 = t.to(torch.bfloat16)
+            if forward_method == "quest":
+                return ops.quantize_quest(t16, group, swizzled=True, return_mask=t.requires_grad)
+            return ops.quantize(t16, "mxfp4", group, None, swizzled=True)[:2] + (None,)
+
+        xq, wq = quantize(x_flat), quantize(weight)
+        y = ops.gemm_fp4(xq[0], wq[0], xq[1], wq[1], constants.alpha, "mxfp4")
+    else:
+        xq = forward_quantize(x_flat, hadamard_matrix, act_global_scale, dtype, forward_method)
+        wq = forward_quantize(weight, hadamard_matrix, weight_global_scale, dtype, forward_method)
+        y = forward_gemm(xq[0], wq[0], xq[1], wq[1], 1.0 / (weight_global_scale * act_global_scale), dtype)
+    y = y.unflatten(dim=0, sizes=x.shape[:-1])
+    if bias is not None:
+        y = y + bias
+    return y, xq, wq, direct
+
+
+def _fused_mxfp4_backward(hadamard_matrix: torch.Tensor, out_features: int) -> bool:
+    """Whether the MXFP4 backward runs on the transposing kernels: a rotation that fits a scale group, rows they can load."""
+    kind, group = kind_of(0, hadamard_matrix.to(torch.bfloat16))
+    return kind in ("hadamard", "identity") and group <= 32 and out_features % 8 == 0
 
 
 class FPQuant4x8MasterFn(Function):
@@ -189,15 +262,10 @@ class FPQuant4x8MasterFn(Function):
 
     @staticmethod
     def forward(ctx, x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype,
-                forward_method):
-        x_flat = x.contiguous().flatten(end_dim=-2)
-        x_q, x_scales, x_mask = forward_quantize(x_flat, forward_hadamard_matrix, act_global_scale, dtype, forward_method)
-        w_q, w_scales, w_mask = forward_quantize(weight, forward_hadamard_matrix, weight_global_scale, dtype, forward_method)
-        y = forward_gemm(x_q, w_q, x_scales, w_scales, 1.0 / (weight_global_scale * act_global_scale), dtype)
-        y = y.unflatten(dim=0, sizes=x.shape[:-1])
-        if bias is not None:
-            y = y + bias
-        ctx.x_shape, ctx.bias_present = x.shape, bias is not None
+                forward_method, constants: Optional[GemmConstants] = None):
+        y, (x_q, x_scales, x_mask), (w_q, w_scales, w_mask), ctx.swizzled = _training_forward(
+            x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype, forward_method, constants)
+        ctx.x_shape, ctx.bias_present, ctx.constants = x.shape, bias is not None, constants
         ctx.masks = (x_mask, w_mask)
         ctx.save_for_backward(x_q, w_q, x_scales, w_scales, act_global_scale, weight_global_scale, forward_hadamard_matrix)
         return y
@@ -207,9 +275,10 @@ class FPQuant4x8MasterFn(Function):
         x_q, w_q, x_scales, w_scales, act_global_scale, weight_global_scale, hadamard_matrix = ctx.saved_tensors
         x_mask, w_mask = ctx.masks
         grad_input, grad_weight = _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale,
-                                                  weight_global_scale, x_mask, w_mask, hadamard_matrix, ctx.x_shape, True)
+                                                  weight_global_scale, x_mask, w_mask, hadamard_matrix, ctx.x_shape, True,
+                                                  ctx.swizzled, ctx.constants)
         grad_bias = grad_output.flatten(end_dim=-2).sum(dim=0) if ctx.bias_present else None
-        return grad_input, grad_weight, None, None, grad_bias, None, None, None
+        return grad_input, grad_weight, None, None, grad_bias, None, None, None, None
 
 
 class FPQuant4x8NoMasterFn(Function):
@@ -239,15 +308,11 @@ class FPQuant4x4MasterFn(Function):
 
     @staticmethod
     def forward(ctx, x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype,
-                forward_method):
-        x_flat = x.contiguous().flatten(end_dim=-2)
-        x_q, x_scales, x_mask = forward_quantize(x_flat, forward_hadamard_matrix, act_global_scale, dtype, forward_method)
-        w_q, w_scales, w_mask = forward_quantize(weight, forward_hadamard_matrix, weight_global_scale, dtype, forward_method)
-        y = forward_gemm(x_q, w_q, x_scales, w_scales, 1.0 / (weight_global_scale * act_global_scale), dtype)
-        y = y.unflatten(dim=0, sizes=x.shape[:-1])
-        if bias is not None:
-            y = y + bias
-        ctx.x_shape, ctx.bias_present = x.shape, bias is not None
+                forward_method, constants: Optional[GemmConstants] = None):
+        y, (x_q, x_scales, x_mask), (w_q, w_scales, w_mask), ctx.swizzled = _training_forward(
+            x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype, forward_method, constants,
+            direct=_fused_mxfp4_backward(forward_hadamard_matrix, weight.shape[0]))
+        ctx.x_shape, ctx.bias_present, ctx.constants = x.shape, bias is not None, constants
         ctx.masks = (x_mask, w_mask)
         ctx.save_for_backward(x_q, w_q, x_scales, w_scales, act_global_scale, weight_global_scale, forward_hadamard_matrix)
         return y
@@ -268,20 +333,23 @@ class FPQuant4x4MasterFn(Function):
         # abs_max MXFP4 carries a factor 3 per operand (the scale is a third of the power of two that is stored)
         ninth = torch.full((1,), 1.0 / 9.0, dtype=torch.float32, device=g.device)
         kind, group = kind_of(0, backward_hadamard_matrix)
-        if kind in ("hadamard", "identity") and group <= 32 and out_features % 8 == 0:
+        if _fused_mxfp4_backward(hadamard_matrix, out_features):
             # Same data flow as the op sequence below with the re-layouts folded into the producers: scales come
             # out in the layout the GEMM reads, the transposes happen inside the (de)quantise kernels, and the
             # token axis is padded to a whole number of K tiles by the kernels that write it.
             gh = group if kind == "hadamard" else 0
-            w_rm = _row_major_scales(w_scales, out_features, in_features // 32)
-            x_rm = _row_major_scales(x_scales, tokens, in_features // 32)
+            swz, consts = ctx.swizzled, ctx.constants
+            w_sc, x_sc = (w_scales, x_scales) if swz else (_row_major_scales(w_scales, out_features, in_features // 32),
+                                                           _row_major_scales(x_scales, tokens, in_features // 32))
+            w_gs, x_gs = (consts.weight_scale, consts.act_scale) if consts is not None else (weight_global_scale.float(),
+                                                                                              act_global_scale.float())
             g_q, g_s, _ = ops.quantize(g, "mxfp4", gh, None, swizzled=True)
-            wt_q, wt_s = ops.mxfp4_requantize_transposed(w_q.view(torch.uint8), w_rm, weight_global_scale.float(), gh,
-                                                         swizzled=True)                                        # [in, out]
+            wt_q, wt_s = ops.mxfp4_requantize_transposed(w_q.view(torch.uint8), w_sc, w_gs, gh, swizzled=True,
+                                                         scales_swizzled=swz)                                     # [in, out]
             grad_input = ops.gemm_fp4(g_q, wt_q, g_s, wt_s, ninth, "mxfp4")
             gt_q, gt_s = ops.quantize_transposed(g, gh, pad_to=128, swizzled=True)                             # [out, tokens_up128]
-            xt_q, xt_s = ops.mxfp4_requantize_transposed(x_q.view(torch.uint8), x_rm, act_global_scale.float(), gh, pad_to=128,
-                                                         swizzled=True)                                        # [in, tokens_up128]
+            xt_q, xt_s = ops.mxfp4_requantize_transposed(x_q.view(torch.uint8), x_sc, x_gs, gh, pad_to=128, swizzled=True,
+                                                         scales_swizzled=swz)                                     # [in, tokens_up128]
             grad_weight = ops.gemm_fp4(gt_q, xt_q, gt_s, xt_s, ninth, "mxfp4")
         else:
             g_q, g_scales, _ = fused_quantize_mx_op(g, backward_hadamard_matrix, "abs_max", False)
@@ -303,4 +371,4 @@ class FPQuant4x4MasterFn(Function):
         grad_input = _unrotate(grad_input, x_mask, hadamard_matrix).view(ctx.x_shape)
         grad_weight = _unrotate(grad_weight, w_mask, hadamard_matrix).view(out_features, in_features)
         grad_bias = g.sum(dim=0) if ctx.bias_present else None
-        return grad_input, grad_weight, None, None, grad_bias, None, None, None
+        return grad_input, grad_weight, None, None, grad_bias, None, None, None, None

@@ -28,7 +28,7 @@ def _cuda(t: torch.Tensor, name: str = "tensor") -> torch.Tensor:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.device.index)     # without building a Stream object (1 us of 1.2)
 
 
 class _NoGuard:
@@ -275,10 +275,11 @@ _error_flags = {}
 
 def device_error_flag(device: torch.device) -> torch.Tensor:
     """int32[1] on `device` that kernels with bounded waits set when a wait ran out."""
-    key = torch.device(device).index or 0
-    if key not in _error_flags:
-        _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-    return _error_flags[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    flag = _error_flags.get(key)
+    if flag is None:
+        flag = _error_flags[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
+    return flag
 
 
 def check_device_errors(device: torch.device) -> None:
@@ -314,6 +315,27 @@ def gemm_fp4(a_codes: torch.Tensor, b_codes: torch.Tensor, a_scales_swizzled: to
     with _guard(a.device):
         C.call("fpq_gemm_fp4", a.data_ptr(), b.data_ptr(), sa.data_ptr(), sb.data_ptr(), alpha.data_ptr(),
                _ptr(bias), out.data_ptr(), M, N, K, FORMATS[fmt], device_error_flag(a.device).data_ptr(), _stream(a))
+    return out
+
+
+def linear_forward(x: torch.Tensor, up: Optional[torch.Tensor], w_codes: torch.Tensor, w_scales_swizzled: torch.Tensor,
+                   alpha: torch.Tensor, fmt: str, hadamard_group: int, quest: bool, global_scale: Optional[torch.Tensor],
+                   bias: Optional[torch.Tensor]) -> torch.Tensor:
+    """quantise + `gemm_fp4` in one call: bf16 [.., N] of x bf16 [.., K] (times silu: `quantize_silu_mul(x, up)`).  The
+    caller vouches for the types: contiguous bf16 x and up of one shape, w_codes u8 [N, K/2], swizzled weight scales,
+    fp32 [1] alpha (and global_scale for NVFP4), bf16 [N] bias or None, all on x's device."""
+    n, k = w_codes.shape[0], x.shape[-1]
+    m = x.numel() // k
+    nv = fmt == "nvfp4"
+    sf_cols = k // 16 if nv else k // 32
+    size = ((m * k // 2 + 255) & -256) + ((m + 127) & -128) * ((sf_cols + 3) & -4)
+    dev = x.device
+    ws = torch.empty(size, dtype=torch.uint8, device=dev)
+    out = torch.empty(x.shape[:-1] + (n,), dtype=torch.bfloat16, device=dev)
+    with _guard(dev):
+        C.call("fpq_linear_forward", x.data_ptr(), _ptr(up), m, n, k, hadamard_group, C.FMT_NVFP4 if nv else C.FMT_MXFP4,
+               quest, global_scale.data_ptr() if nv else None, w_codes.data_ptr(), w_scales_swizzled.data_ptr(),
+               alpha.data_ptr(), _ptr(bias), ws.data_ptr(), size, out.data_ptr(), device_error_flag(dev).data_ptr(), _stream(x))
     return out
 
 
@@ -375,21 +397,24 @@ def quantize_mxfp8_square(x: torch.Tensor, swizzled: bool = False, transposed: b
     return (out, rs, cs, out_t) if transposed else (out, rs, cs)
 
 
-def mxfp4_transpose_mxfp8(codes: torch.Tensor, scales_rowmajor: torch.Tensor, swizzled: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
-    """MXFP4 (codes u8 [rows, cols/2], E8M0 bytes [rows, cols/32], row-major, unpadded) -> the transpose as
-    MXFP8: (E4M3 [cols, rows_pad], scales u8 [cols, rows_pad/32], swizzled for the GEMM on request)."""
+def mxfp4_transpose_mxfp8(codes: torch.Tensor, scales_rowmajor: torch.Tensor, swizzled: bool = False,
+                          scales_swizzled: bool = False) -> Tuple[torch.Tensor, torch.Tensor]:
+    """MXFP4 (codes u8 [rows, cols/2], E8M0 bytes [rows, cols/32], row-major and unpadded or, with `scales_swizzled`, in
+    the swizzled layout) -> the transpose as MXFP8: (E4M3 [cols, rows_pad], scales u8 [cols, rows_pad/32], swizzled for the
+    GEMM on request)."""
     codes = _cuda(codes, "codes").contiguous()
     sc = _cuda(scales_rowmajor, "scales")
     sc = (sc if sc.dtype == torch.uint8 else sc.view(torch.uint8)).contiguous()
     rows, cols = codes.shape[0], codes.shape[1] * 2
-    if tuple(sc.shape) != (rows, cols // 32):
+    if tuple(sc.shape) != (padded_scale_shape(rows, cols // 32) if scales_swizzled else (rows, cols // 32)):
         raise ValueError(f"scales must be [{rows}, {cols // 32}] row-major bytes, got {tuple(sc.shape)}")
     rp = (rows + 127) // 128 * 128
     out = torch.empty(cols, rp, dtype=torch.float8_e4m3fn, device=codes.device)
     os_ = _scale_buffer(cols, rp // 32, swizzled, codes.device)
+    layout = (C.SCALES_SWIZZLED if swizzled else C.SCALES_ROWMAJOR) | (C.SCALES_INPUT_SWIZZLED if scales_swizzled else 0)
     with _guard(codes.device):
         C.call("fpq_mxfp4_transpose_mxfp8", codes.data_ptr(), sc.data_ptr(), rows, cols, out.data_ptr(), os_.data_ptr(),
-               C.SCALES_SWIZZLED if swizzled else C.SCALES_ROWMAJOR, _stream(codes))
+               layout, _stream(codes))
     return out, os_
 
 

@@ -36,6 +36,7 @@ extern "C" {
 
 /* layouts of the scale bytes */
 #define FPQ_SCALES_ROWMAJOR 0 /* [rows, cols/g] */
+#define FPQ_SCALES_INPUT_SWIZZLED 16 /* flag for fpq_mxfp4_transpose_mxfp8: its input scales are swizzled too */
 #define FPQ_SCALES_SWIZZLED 1 /* 128x4 tiles, padded to [ceil(rows/128)*128, ceil(cols/g/4)*4] */
 
 /* what fpq_apply_scales writes */
@@ -282,6 +283,19 @@ int fpq_quantize_transposed(const void* x_bf16, int64_t t_rows, int64_t n, int64
 int fpq_mxfp4_requantize_transposed(const uint8_t* codes_in, const uint8_t* scales_in, int scale_layout_in,
                                     const float* alpha, int64_t t_rows, int64_t n, int64_t t_pad, int hadamard_group,
                                     uint8_t* codes, uint8_t* scale_bytes, int scale_layout, fpq_stream_t stream);
+
+/*
+ * The forward pass of a quantised linear layer in one call (FPQuant4x16NoMasterFn.forward,
+ * inference_lib/src/fp_quant/module/linear_fns.py:484-528): fpq_quantize (or fpq_quantize_quest, or with up_bf16
+ * fpq_quantize_silu_mul of gate = x) into `workspace`, then fpq_gemm_fp4.  x, up: bf16 [M, K]; out: bf16 [M, N].
+ * workspace: fpq_linear_workspace_bytes bytes, 256-byte aligned; holds the codes and scale bytes of x until the
+ * kernels have run.
+ */
+int64_t fpq_linear_workspace_bytes(int64_t M, int64_t K, int format);
+int fpq_linear_forward(const void* x_bf16, const void* up_bf16, int64_t M, int64_t N, int64_t K, int hadamard_group,
+                       int format, int quest, const float* global_scale, const uint8_t* w_codes,
+                       const uint8_t* w_scales_swizzled, const float* alpha, const void* bias_bf16, void* workspace,
+                       int64_t workspace_bytes, void* out_bf16, int32_t* error_flag, fpq_stream_t stream);
 
 /*
  * Column-parallel form of fpq_gemm_fp4 for tensor parallelism over NVLink (no counterpart in the reference,
