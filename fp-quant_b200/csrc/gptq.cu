@@ -94,106 +94,306 @@ __global__ void reflect_inplace_kernel(float* A, int64_t d) {
 // L^-1 (lower) to Linv.  A non-positive or non-finite pivot sets *status and is replaced by 1 so
 // that the kernel always terminates with finite data.
 //
-// Both matrices live in registers: the 256 threads form a 16 x 16 grid, thread (ty, tx) owns the
-// entries (ty + 16 r, tx + 16 c), r, c = 0..7, of A and of X (X starts as the identity).  Step k
-// is one right-looking elimination step applied to both: column k of A and row k of X go through
-// shared memory (double buffered, so one barrier per step), then
-//     L[:, k] = A[:, k] / sqrt(A[k, k]),    X[k, :] /= L[k, k],
-//     A[i, j] -= L[i, k] L[j, k]  (i, j > k),    X[i, :] -= L[i, k] X[k, :]  (i > k).
-// The loop over the register index k / 16 is unrolled so that every register index is static;
-// register blocks that are already final (or still zero) are skipped at compile time.
-__global__ void __launch_bounds__(256) chol_diag_kernel(float* A, int64_t lda, float* Linv, int64_t ldi, int nb,
+// The kernel is one chain of dependent steps, so it is laid out for a short chain: blocks of 32 columns in shared
+// memory.  A block's 32 x 32 diagonal part is factored by one warp, a row per lane, in registers; a step costs one
+// shuffle latency (the pivot and the whole column leave together, unscaled: A[i, j] -= c_i c_j / pivot), a reciprocal
+// and a fused multiply-add, no barrier.  Everything else is done by many threads at a time and meanwhile:
+//   phase 1   warp 0 factors D_p
+//   phase 2   warps 0-3: the rows below and D_p^-1   | warps 4-7: S_p = L_(p, <p) X_(<p)
+//             (one forward substitution per thread)  |
+//   phase 3   all: X_p = -D_p^-1 S_p, the trailing part -= L L^T
+// with X = L^-1 by blocks of rows.  128 x 128: 35 us; 48 us as one right-looking elimination with a barrier per column.
+constexpr int CD_LD = NB + 4;         // row stride in shared memory: 16-byte rows whose starts walk through the banks
+constexpr int CD_B = 32;              // block of columns
+constexpr int CD_SLD = 96 + 4;
+constexpr int CD_SMEM = (2 * NB * CD_LD + CD_B * CD_SLD + NB) * (int)sizeof(float);
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return *reinterpret_cast<float2*>(&r);
+}
+
+// Factor the 32 x 32 block at D in place (lower part; the upper part becomes zero), 1 / L[k, k] to rd.
+__device__ __forceinline__ void factor32(float* D, float* rd, int lane, int32_t* status) {
+  float a[CD_B];
+#pragma unroll
+  for (int q = 0; q < CD_B / 4; ++q) {
+    const float4 v = *reinterpret_cast<const float4*>(D + lane * CD_LD + 4 * q);
+    a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
+  }
+  bool bad = false;
+  float mine = 1.0f;                                       // this row's pivot
+#pragma unroll
+  for (int k = 0; k < CD_B; ++k) {
+    const float c = a[k];
+    float piv = __shfl_sync(0xffffffffu, c, k);
+    const bool ok = piv >= 1.17549435e-38f && piv <= 3.40282347e38f;
+    piv = ok ? piv : 1.0f;
+    bad |= !ok;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
+    const float t0 = c * r;
+    const float t = fmaf(t0, fmaf(-piv, r, 1.0f), t0);     // one Newton step: c / pivot with full fp32 accuracy
+    // rows at or above k get values that nothing reads
+#pragma unroll
+    for (int j = k + 1; j < CD_B; ++j) a[j] = fmaf(-t, __shfl_sync(0xffffffffu, c, j), a[j]);
+    if (lane == k) {
+      mine = piv;
+      a[k] = piv;
+    }
+  }
+  // the square roots wait until here, off the chain: column k is divided by sqrt(pivot k)
+  float rinv = rsqrtf(mine);
+  rinv = rinv * fmaf(-0.5f * mine * rinv, rinv, 1.5f);
+#pragma unroll
+  for (int k = 0; k < CD_B; ++k) a[k] *= __shfl_sync(0xffffffffu, rinv, k);
+  if (bad && lane == 0) atomicExch(status, 1);
+  rd[lane] = rinv;
+#pragma unroll
+  for (int q = 0; q < CD_B / 4; ++q) {
+    float4 v;
+    v.x = 4 * q <= lane ? a[4 * q] : 0.0f;
+    v.y = 4 * q + 1 <= lane ? a[4 * q + 1] : 0.0f;
+    v.z = 4 * q + 2 <= lane ? a[4 * q + 2] : 0.0f;
+    v.w = 4 * q + 3 <= lane ? a[4 * q + 3] : 0.0f;
+    *reinterpret_cast<float4*>(D + lane * CD_LD + 4 * q) = v;
+  }
+}
+
+// v <- L^-1 v for the 32 x 32 lower block at L (every thread a right-hand side of its own; L is read as a broadcast).
+__device__ __forceinline__ void solve32(const float* L, const float* rd, float (&v)[CD_B]) {
+#pragma unroll
+  for (int k = 0; k < CD_B; ++k) {
+    float s = v[k];
+#pragma unroll
+    for (int q = 0; q < CD_B / 4; ++q) {
+      if (4 * q >= k) continue;
+      const float4 l = *reinterpret_cast<const float4*>(L + k * CD_LD + 4 * q);
+      s = fmaf(-l.x, v[4 * q], s);
+      if (4 * q + 1 < k) s = fmaf(-l.y, v[4 * q + 1], s);
+      if (4 * q + 2 < k) s = fmaf(-l.z, v[4 * q + 2], s);
+      if (4 * q + 3 < k) s = fmaf(-l.w, v[4 * q + 3], s);
+    }
+    v[k] = s * rd[k];
+  }
+}
+
+// A[r0 + i, r0 + j] -= sum_k P[i, k] P[j, k] over the T x T sixteenths below (and on) the diagonal; P = 32 columns.
+template <int T>
+__device__ __forceinline__ void trailing32(float* A, int r0, int c0, int ty, int tx) {
+  float2 acc[T][T];
+#pragma unroll
+  for (int r = 0; r < T; ++r)
+#pragma unroll
+    for (int c = 0; c < T; ++c) acc[r][c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int q = 0; q < CD_B / 4; ++q) {
+    float4 pi[T], pj[T];
+#pragma unroll
+    for (int r = 0; r < T; ++r) {
+      pi[r] = *reinterpret_cast<const float4*>(A + (r0 + ty + 16 * r) * CD_LD + c0 + 4 * q);
+      pj[r] = *reinterpret_cast<const float4*>(A + (r0 + tx + 16 * r) * CD_LD + c0 + 4 * q);
+    }
+#pragma unroll
+    for (int r = 0; r < T; ++r)
+#pragma unroll
+      for (int c = 0; c <= r; ++c) {
+        acc[r][c] = fma2(make_float2(pi[r].x, pi[r].y), make_float2(pj[c].x, pj[c].y), acc[r][c]);
+        acc[r][c] = fma2(make_float2(pi[r].z, pi[r].w), make_float2(pj[c].z, pj[c].w), acc[r][c]);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < T; ++r)
+#pragma unroll
+    for (int c = 0; c <= r; ++c) A[(r0 + ty + 16 * r) * CD_LD + r0 + tx + 16 * c] -= acc[r][c].x + acc[r][c].y;
+}
+
+// X rows [32 p, 32 p + 32), columns left of the diagonal block: -X_pp S.  Eight threads a row, four columns of every block.
+__device__ __forceinline__ void inverse_row(float* __restrict__ X, const float* __restrict__ S, int p, int tid) {
+  const int row = tid >> 3, col = (tid & 7) * 4;
+  const float* D = X + (32 * p + row) * CD_LD + 32 * p;
+  float2 d[CD_B / 2];
+#pragma unroll
+  for (int q = 0; q < CD_B / 4; ++q) {
+    const float4 v = *reinterpret_cast<const float4*>(D + 4 * q);
+    d[2 * q] = make_float2(-v.x, -v.y);
+    d[2 * q + 1] = make_float2(-v.z, -v.w);
+  }
+  for (int jb = 0; jb < p; ++jb) {
+    float2 lo = make_float2(0.0f, 0.0f), hi = lo;
+#pragma unroll
+    for (int k = 0; k < CD_B; ++k) {                       // D is zero beyond k = row
+      const float dk = (k & 1) ? d[k / 2].y : d[k / 2].x;
+      const float4 sv = *reinterpret_cast<const float4*>(S + k * CD_SLD + jb * CD_B + col);
+      lo = fma2(make_float2(dk, dk), make_float2(sv.x, sv.y), lo);
+      hi = fma2(make_float2(dk, dk), make_float2(sv.z, sv.w), hi);
+    }
+    *reinterpret_cast<float4*>(X + (32 * p + row) * CD_LD + jb * CD_B + col) = make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
+}
+
+__global__ void __launch_bounds__(256, 1) chol_diag_kernel(float* A, int64_t lda, float* Linv, int64_t ldi, int nb,
                                                         int32_t* status) {
-  // Column k of A and row k of X as the threads need them: entry i sits at perm(i), so that the eight
-  // values of a thread (i = t + 16 c) are two contiguous groups of four: perm(i) = (c / 4) * 64 + t * 4 + c % 4.
-  __shared__ __align__(16) float colbuf[2][NB];
-  __shared__ __align__(16) float rowbuf[2][NB];
-  const int tid = threadIdx.x;
-  const int ty = tid >> 4, tx = tid & 15;
-  float a[8][8], x[8][8];
+  extern __shared__ __align__(16) float cd_smem[];
+  float* As = cd_smem;
+  float* X = As + NB * CD_LD;
+  float* S = X + NB * CD_LD;
+  float* rd = S + CD_B * CD_SLD;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool vec = nb == NB && lda % 4 == 0 && ldi % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)Linv & 15) == 0;
+  for (int o = tid; o < NB * NB / 4; o += 256) {
+    const int i = o / (NB / 4), j = (o % (NB / 4)) * 4;
+    float v[4];
+    if (vec) {
+      *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(A + (int64_t)i * lda + j);
+    } else {
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
+      for (int q = 0; q < 4; ++q) v[q] = (i < nb && j + q < nb) ? A[(int64_t)i * lda + j + q] : (i == j + q ? 1.0f : 0.0f);
+    }
+    *reinterpret_cast<float4*>(As + i * CD_LD + j) = *reinterpret_cast<float4*>(v);
+    *reinterpret_cast<float4*>(X + i * CD_LD + j) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int p = 0; p < NB / CD_B; ++p) {
+    const int c0 = CD_B * p, below = NB - c0 - CD_B;
+    float* D = As + c0 * CD_LD + c0;
+    if (warp == 0) factor32(D, rd + c0, lane, status);
+    __syncthreads();
+    if (warp < 4) {
+      // right-hand sides: the rows below, then (last warp) the unit vectors, whose solutions are the columns of D^-1
+      const bool unit = warp == 3;
+      if (unit || tid < below) {
+        float v[CD_B];
+        float* row = As + (c0 + CD_B + tid) * CD_LD + c0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int i = ty + 16 * r, j = tx + 16 * c;
-      a[r][c] = (i < nb && j < nb) ? A[(int64_t)i * lda + j] : (i == j ? 1.0f : 0.0f);
-      x[r][c] = i == j ? 1.0f : 0.0f;
+        for (int q = 0; q < CD_B / 4; ++q) {
+          float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (!unit) w = *reinterpret_cast<const float4*>(row + 4 * q);
+          v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+        }
+        if (unit) {
+#pragma unroll
+          for (int k = 0; k < CD_B; ++k) v[k] = lane == k ? 1.0f : 0.0f;
+        }
+        solve32(D, rd + c0, v);
+        if (unit) {
+#pragma unroll
+          for (int k = 0; k < CD_B; ++k) X[(c0 + k) * CD_LD + c0 + lane] = v[k];
+        } else {
+#pragma unroll
+          for (int q = 0; q < CD_B / 4; ++q)
+            *reinterpret_cast<float4*>(row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+      }
+    } else if (p > 0) {
+      // S = L[c0 .. c0 + 31, 0 .. c0 - 1] X[0 .. c0 - 1, 0 .. c0 - 1], X lower triangular by blocks
+      const int t = tid - 128, r = t >> 2, cq = (t & 3) * 4;
+      const float* Lr = As + (c0 + r) * CD_LD;
+      for (int jb = 0; jb < p; ++jb) {
+        const int j = jb * CD_B + cq;                      // columns j .. j + 3 and j + 16 .. j + 19
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0, s2 = s0, s3 = s0;
+#pragma unroll 8
+        for (int k = jb * CD_B; k < c0; ++k) {
+          const float2 l = make_float2(Lr[k], Lr[k]);
+          const float4 x0 = *reinterpret_cast<const float4*>(X + k * CD_LD + j);
+          const float4 x1 = *reinterpret_cast<const float4*>(X + k * CD_LD + j + 16);
+          s0 = fma2(l, make_float2(x0.x, x0.y), s0);
+          s1 = fma2(l, make_float2(x0.z, x0.w), s1);
+          s2 = fma2(l, make_float2(x1.x, x1.y), s2);
+          s3 = fma2(l, make_float2(x1.z, x1.w), s3);
+        }
+        *reinterpret_cast<float4*>(S + r * CD_SLD + j) = make_float4(s0.x, s0.y, s1.x, s1.y);
+        *reinterpret_cast<float4*>(S + r * CD_SLD + j + 16) = make_float4(s2.x, s2.y, s3.x, s3.y);
+      }
+    }
+    __syncthreads();
+    if (p > 0) inverse_row(X, S, p, tid);
+    if (p == 0) trailing32<6>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
+    if (p == 1) trailing32<4>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
+    if (p == 2) trailing32<2>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
+    __syncthreads();
+  }
+  for (int o = tid; o < NB * NB / 4; o += 256) {
+    const int i = o / (NB / 4), j = (o % (NB / 4)) * 4;
+    float a[4], x[4];
+    *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(As + i * CD_LD + j);
+    *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(X + i * CD_LD + j);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (j + q > i) a[q] = 0.0f;                          // above the diagonal: what the updates left there
+    if (vec) {
+      *reinterpret_cast<float4*>(A + (int64_t)i * lda + j) = *reinterpret_cast<float4*>(a);
+      *reinterpret_cast<float4*>(Linv + (int64_t)i * ldi + j) = *reinterpret_cast<float4*>(x);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i < nb && j + q < nb) {
+          A[(int64_t)i * lda + j + q] = a[q];
+          Linv[(int64_t)i * ldi + j + q] = x[q];
+        }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ panel below a diagonal block
+// A[i, 0..127] <- sum_k A[i, k] Linv[j, k] (k <= j) in place for `rows` rows: L21 = A21 L11^-T.  A CTA takes 32 rows, so
+// that even a short panel spreads over the SMs, and holds Linv in shared memory; a thread has 2 x 8 outputs, the part
+// of Linv above its diagonal is skipped.  Latency-bound; as a 128 x 128-tile matrix product on at most 112 CTAs it took
+// 18 to 20 us a panel on average, here 10 (d = 4096) to 15 (d = 14336).
+constexpr int PANEL_ROWS = 32;
+constexpr int PANEL_SMEM = (NB + PANEL_ROWS) * CD_LD * (int)sizeof(float);
+
+__global__ void __launch_bounds__(256, 2) chol_panel_kernel(float* A, int64_t lda, int64_t rows, const float* __restrict__ Linv,
+                                                            int64_t ldi) {
+  extern __shared__ __align__(16) float pn_smem[];
+  float* Ls = pn_smem;
+  float* Ps = Ls + NB * CD_LD;
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int64_t r0 = (int64_t)blockIdx.x * PANEL_ROWS;
+  const bool vec = lda % 4 == 0 && ldi % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)Linv & 15) == 0;
+  for (int o = tid; o < (NB + PANEL_ROWS) * NB / 4; o += 256) {
+    const int i = o / (NB / 4), j = (o % (NB / 4)) * 4;
+    const bool is_l = i < NB;
+    const int64_t ar = r0 + i - NB;
+    const float* src = is_l ? Linv + (int64_t)i * ldi + j : A + ar * lda + j;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (is_l || ar < rows) v = vec ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+    *reinterpret_cast<float4*>((is_l ? Ls + i * CD_LD : Ps + (i - NB) * CD_LD) + j) = v;
+  }
+  __syncthreads();
+  float2 acc[2][8];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[r][c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int kb = 0; kb < 8; ++kb) {                         // sixteen k at a time: columns tx + 16 c with c >= kb need them
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = 16 * kb + 4 * q;
+      const float4 a0 = *reinterpret_cast<const float4*>(Ps + ty * CD_LD + k);
+      const float4 a1 = *reinterpret_cast<const float4*>(Ps + (ty + 16) * CD_LD + k);
+#pragma unroll
+      for (int c = kb; c < 8; ++c) {
+        const float4 l = *reinterpret_cast<const float4*>(Ls + (tx + 16 * c) * CD_LD + k);
+        acc[0][c] = fma2(make_float2(a0.x, a0.y), make_float2(l.x, l.y), acc[0][c]);
+        acc[0][c] = fma2(make_float2(a0.z, a0.w), make_float2(l.z, l.w), acc[0][c]);
+        acc[1][c] = fma2(make_float2(a1.x, a1.y), make_float2(l.x, l.y), acc[1][c]);
+        acc[1][c] = fma2(make_float2(a1.z, a1.w), make_float2(l.z, l.w), acc[1][c]);
+      }
     }
   }
 #pragma unroll
-  for (int cc = 0; cc < 8; ++cc) {
-    for (int t = 0; t < 16; ++t) {
-      const int k = 16 * cc + t;
-      float* cb = colbuf[k & 1];
-      float* rb = rowbuf[k & 1];
-      if (tx == t) {
+  for (int r = 0; r < 2; ++r) {
+    const int64_t row = r0 + ty + 16 * r;
+    if (row >= rows) continue;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) cb[(r >> 2) * 64 + ty * 4 + (r & 3)] = a[r][cc];
-      }
-      if (ty == t) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) rb[(c >> 2) * 64 + tx * 4 + (c & 3)] = x[cc][c];
-      }
-      __syncthreads();
-      float piv = cb[(cc >> 2) * 64 + t * 4 + (cc & 3)];
-      if (!(piv > 0.0f) || !isfinite(piv)) {
-        if (tid == 0) atomicExch(status, 1);
-        piv = 1.0f;
-      }
-      // The updates need only 1 / pivot: with c = A[:, k] and y = X[k, :] (both unscaled),
-      //   A[i, j] -= c_i c_j / piv,   X[i, :] -= c_i y / piv;
-      // the square root is taken off the critical path, by the owners of column k / row k alone.
-      const float pinv = __frcp_rn(piv);
-      float li[8], lj[8], xr[8];
-      {
-        const float4 v0 = *reinterpret_cast<const float4*>(&cb[ty * 4]), v1 = *reinterpret_cast<const float4*>(&cb[64 + ty * 4]);
-        li[0] = v0.x; li[1] = v0.y; li[2] = v0.z; li[3] = v0.w; li[4] = v1.x; li[5] = v1.y; li[6] = v1.z; li[7] = v1.w;
-        const float4 w0 = *reinterpret_cast<const float4*>(&cb[tx * 4]), w1 = *reinterpret_cast<const float4*>(&cb[64 + tx * 4]);
-        lj[0] = w0.x; lj[1] = w0.y; lj[2] = w0.z; lj[3] = w0.w; lj[4] = w1.x; lj[5] = w1.y; lj[6] = w1.z; lj[7] = w1.w;
-        const float4 y0 = *reinterpret_cast<const float4*>(&rb[tx * 4]), y1 = *reinterpret_cast<const float4*>(&rb[64 + tx * 4]);
-        xr[0] = y0.x; xr[1] = y0.y; xr[2] = y0.z; xr[3] = y0.w; xr[4] = y1.x; xr[5] = y1.y; xr[6] = y1.z; xr[7] = y1.w;
-      }
-      float ljs[8], xrs[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        ljs[c] = lj[c] * pinv;
-        xrs[c] = xr[c] * pinv;
-      }
-      const bool below = ty > t;   // row ty + 16 cc lies below row k
-#pragma unroll
-      for (int r = cc; r < 8; ++r) {
-        if (r > cc || below) {
-#pragma unroll
-          for (int c = cc; c < 8; ++c)
-            if (c > cc || tx > t) a[r][c] = fmaf(-li[r], ljs[c], a[r][c]);
-#pragma unroll
-          for (int c = 0; c <= cc; ++c) x[r][c] = fmaf(-li[r], xrs[c], x[r][c]);
-        }
-      }
-      if (tx == t || ty == t) {
-        float rinv = rsqrtf(piv);
-        rinv = rinv * fmaf(-0.5f * piv * rinv, rinv, 1.5f);   // one Newton step: full fp32 accuracy
-        if (tx == t) {
-#pragma unroll
-          for (int r = cc; r < 8; ++r) a[r][cc] = li[r] * rinv;
-        }
-        if (ty == t) {
-#pragma unroll
-          for (int c = 0; c <= cc; ++c) x[cc][c] = xr[c] * rinv;
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int i = ty + 16 * r, j = tx + 16 * c;
-      if (i < nb && j < nb) {
-        A[(int64_t)i * lda + j] = j <= i ? a[r][c] : 0.0f;
-        Linv[(int64_t)i * ldi + j] = j <= i ? x[r][c] : 0.0f;
-      }
-    }
+    for (int c = 0; c < 8; ++c) A[row * lda + tx + 16 * c] = acc[r][c].x + acc[r][c].y;
   }
 }
 
@@ -678,6 +878,14 @@ extern "C" int fpq_cholesky_inverse_upper(const float* H, float* U, int64_t d, f
   float* L = workspace;
   float* scratch = workspace + ((d * d + 3) & ~(int64_t)3);
   __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(scratch + half * half);
+  static bool configured[64] = {};
+  int dev = 0;
+  FPQ_CHECK_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !configured[dev]) {
+    FPQ_CHECK_CUDA(cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CD_SMEM));
+    FPQ_CHECK_CUDA(cudaFuncSetAttribute(chol_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM));
+    if (dev < 64) configured[dev] = true;
+  }
   FPQ_CHECK_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), st));
   reverse_copy_kernel<<<grid1d(d * d), 256, 0, st>>>(H, L, d);
   FPQ_CHECK_LAUNCH();
@@ -694,17 +902,14 @@ extern "C" int fpq_cholesky_inverse_upper(const float* H, float* U, int64_t d, f
     for (int k = ob; k < nblk && k < ob + OB; ++k) {
       const int64_t r = (int64_t)k * NB;
       const int nb = (int)((d - r) < NB ? (d - r) : NB);
-      chol_diag_kernel<<<1, 256, 0, st>>>(L + r * d + r, d, U + r * d + r, d, nb, status);
+      chol_diag_kernel<<<1, 256, CD_SMEM, st>>>(L + r * d + r, d, U + r * d + r, d, nb, status);
       FPQ_CHECK_LAUNCH();
       const int64_t below = d - (r + nb);
       if (below <= 0) break;
-      SgemmArgs a{};
-      // panel: L21 = A21 * L11^-T  (in place: every CTA reads only the 128 rows it then overwrites)
-      a.A = L + (r + nb) * d + r; a.lda = d;
-      a.B = U + r * d + r; a.ldb = d;
-      a.C = L + (r + nb) * d + r; a.ldc = d;
-      a.M = (int)below; a.N = nb; a.K = nb; a.alpha = 1.0f; a.beta = 0.0f;
-      if (int rc = sgemm(a, true, SGEMM_PLAIN, st)) return rc;
+      // panel: L21 = A21 L11^-T, in place (a block with rows below it is a whole one)
+      chol_panel_kernel<<<(unsigned)((below + PANEL_ROWS - 1) / PANEL_ROWS), 256, PANEL_SMEM, st>>>(
+          L + (r + nb) * d + r, d, below, U + r * d + r, d);
+      FPQ_CHECK_LAUNCH();
       // inner update: columns [r + nb, R + Wd) of the rows below -= L21 * (the first rows of L21)^T
       const int64_t inner = R + Wd - (r + nb);
       if (inner <= 0) continue;
@@ -715,6 +920,7 @@ extern "C" int fpq_cholesky_inverse_upper(const float* H, float* U, int64_t d, f
           return rc;
         continue;
       }
+      SgemmArgs a{};
       a.A = L + (r + nb) * d + r; a.lda = d;
       a.B = L + (r + nb) * d + r; a.ldb = d;
       a.C = Cin; a.ldc = d;

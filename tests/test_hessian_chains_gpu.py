@@ -43,3 +43,30 @@ def test_output_rows_off_the_vector_alignment(cuda_device):
     assert int(status) == 0
     r = U.double().t() @ (U.double() @ H.double()) - torch.eye(d, device=cuda_device, dtype=torch.float64)
     assert r.abs().max().item() < 1e-3
+
+
+@pytest.mark.parametrize("d", [1, 31, 33, 127, 128, 129, 160, 257, 300, 640, 1100])
+def test_factor_at_block_edges(cuda_device, d):
+    """U = chol(H^-1, upper) where the 128-blocks, the 32-column blocks inside them and the 32-row panels end raggedly.  The
+    chain is backward stable: with a condition number of a few hundred and d eps = 7e-5 at most, 1e-4 relative holds with room."""
+    from fpq_b200 import ops
+
+    x = torch.randn(2 * d + 8, d, device=cuda_device, dtype=torch.float64, generator=torch.Generator(device=cuda_device).manual_seed(d))
+    H = x.t() @ x / (2 * d)
+    H.diagonal().add_(0.05)
+    U, status = ops.cholesky_inverse_upper(H.float())
+    want = torch.linalg.cholesky(torch.linalg.inv(H.float().double()), upper=True)
+    ops.check_device_errors(cuda_device)
+    assert int(status) == 0 and not bool(torch.tril(U, -1).any())
+    assert ((U.double() - want).norm() / want.norm()).item() < 1e-4
+
+
+def test_bad_pivots_are_reported(cuda_device):
+    from fpq_b200 import ops
+
+    for i, v in ((0, 0.0), (40, -1.0), (127, float("nan")), (130, float("inf"))):
+        H = torch.eye(200, device=cuda_device)
+        H[i, i] = v
+        U, status = ops.cholesky_inverse_upper(H)
+        assert int(status) == 1
+    ops.check_device_errors(cuda_device)
