@@ -115,9 +115,12 @@ __device__ __forceinline__ void tile_coords(const HessParams& p, int tile, int& 
 constexpr int BAND = 8;
 __host__ __device__ inline int lower_tiles(int rows) { return rows * (rows + 1) / 2; }
 
-__host__ __device__ inline void pair_tile_coords(int num_blocks, int num_blocks_n, bool symmetric, int tile, int& ib,
-                                                 int& jb) {
-  if (!symmetric) {
+// A lower triangular A^T (tri = 2) gives its last block rows the longest sums: they come first.  (A lower triangular B
+// does so for the first columns, which every band starts with.)
+__device__ __forceinline__ void pair_tile_coords(const HessParams& p, int tile, int& ib, int& jb) {
+  const int num_blocks = p.num_blocks, num_blocks_n = p.num_blocks_n;
+  if (p.tri == 2) tile = p.num_tiles - 1 - tile;
+  if (!p.symmetric) {
     const int b = tile / (BAND * num_blocks_n), left = num_blocks - b * BAND, rows = left < BAND ? left : BAND;
     const int rem = tile - b * BAND * num_blocks_n;
     jb = rem / rows;
@@ -141,11 +144,11 @@ __host__ __device__ inline void pair_tile_coords(int num_blocks, int num_blocks_
 }
 
 // Stages [lo, hi) of every K segment that can contribute to tile (ib, jb2).
-__device__ __forceinline__ void stage_range(const HessParams& p, int ib, int jb2, int& lo, int& hi) {
+__device__ __forceinline__ void stage_range(const HessParams& p, int tile_rows, int ib, int jb2, int& lo, int& hi) {
   lo = 0;
   hi = p.seg_stages;
   if (p.tri == 1) lo = min(jb2 * (TILE_N / BK), p.seg_stages - 1);
-  if (p.tri == 2) hi = max(1, min(p.seg_stages, (ib + 1) * (TILE / BK)));
+  if (p.tri == 2) hi = max(1, min(p.seg_stages, (ib + 1) * (tile_rows / BK)));
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -204,7 +207,7 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         int ib, jb;
         tile_coords(p, tile, ib, jb);
         int lo, hi;
-        stage_range(p, ib, jb, lo, hi);
+        stage_range(p, TILE, ib, jb, lo, hi);
         const int per_seg = hi - lo, n_st = per_seg * p.n_seg;
         for (int ks = 0; ks < n_st; ++ks, ++it) {
           const int s = it % STAGES;
@@ -244,7 +247,7 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         const uint32_t acc = tmem_base + buf * TILE_N;
         int ib, jb, lo, hi;
         tile_coords(p, tile, ib, jb);
-        stage_range(p, ib, jb, lo, hi);
+        stage_range(p, TILE, ib, jb, lo, hi);
         const int n_st = (hi - lo) * p.n_seg;
         // one barrier wait, four MMAs and one commit per stage: every other instruction here is time the
         // tensor pipe idles (the operands come through TMA, which needs no tcgen05 fence)
@@ -438,8 +441,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       bool ok = true;
       for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
         int ib, jb, lo, hi;
-        pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
-        stage_range(p, ib, jb, lo, hi);
+        pair_tile_coords(p, tile, ib, jb);
+        stage_range(p, 256, ib, jb, lo, hi);
         const int per_seg = hi - lo, n_st = per_seg * p.n_seg;
         const int xa = p.a_x0 + ib * 256 + (int)rank * 128, xb = p.b_x0 + jb * TILE_N + (int)rank * 128;
         for (int ks = 0; ks < n_st; ++ks, ++it) {
@@ -477,8 +480,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       bool ok = true;
       for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
         int ib, jb, lo, hi;
-        pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
-        stage_range(p, ib, jb, lo, hi);
+        pair_tile_coords(p, tile, ib, jb);
+        stage_range(p, 256, ib, jb, lo, hi);
         const int n_st = (hi - lo) * p.n_seg;
         for (int k0 = 0; k0 < n_st && ok; k0 += p.chain_stages, ++chain_count) {
           const int k1 = min(n_st, k0 + p.chain_stages);
@@ -516,8 +519,8 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     bool ok = true;
     for (int tile = pair_id; tile < p.num_tiles && ok; tile += num_pairs) {
       int ib, jb, lo, hi;
-      pair_tile_coords(p.num_blocks, p.num_blocks_n, p.symmetric, tile, ib, jb);
-      stage_range(p, ib, jb, lo, hi);
+      pair_tile_coords(p, tile, ib, jb);
+      stage_range(p, 256, ib, jb, lo, hi);
       const int n_st = (hi - lo) * p.n_seg;
       const int rb = ib * 2 + (int)rank;                     // my 128-row block
       const int jblock = jb * 2 + half;                      // my 128-column block
@@ -606,6 +609,16 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
 namespace fpq {
 
+// Whether gemm_atb_bf16 runs a product on CTA pairs: enough 256 x 256 tiles to fill the GPU, eight stages of K or more
+// (measured with the threshold at 64, 24 and 8 stages: the d = 14336 Cholesky-inverse chain 25.7, 25.0, 24.9 ms; with the
+// triangular products of its inverse on pairs as well, whose launches took 8.3 ms on single CTAs: 7.6).
+bool gemm_atb_on_pairs(int64_t d1, int64_t d2, bool symmetric, int n_seg, int64_t seg_rows) {
+  const int64_t total_stages = (int64_t)n_seg * ((seg_rows + BK - 1) / BK);
+  const int64_t rows256 = (d1 + 255) / 256, cols256 = (d2 + TILE_N - 1) / TILE_N;
+  const int64_t tiles = symmetric ? rows256 * (rows256 + 1) / 2 : rows256 * cols256;
+  return total_stages >= 8 && tiles >= sm_count() / 2 && sm_count() >= 2;
+}
+
 // out[d1, d2] (row stride ldc) = beta * out + alpha * A^T B with A [*, d1] and B [*, d2] bf16 row-major
 // matrices of a_rows / b_rows rows (row strides lda, ldb in elements; the operands start at columns
 // a_x0 / b_x0).  The K dimension is the concatenation of n_seg segments of seg_rows rows each, segment
@@ -613,9 +626,10 @@ namespace fpq {
 // With more than one segment seg_rows must be a multiple of 64.  symmetric: only tiles that touch the
 // lower triangle are computed (d1 == d2); mirror: the blocks below the diagonal are also written
 // transposed.  tri = 1: B (as the [K, d2] matrix of one segment) is lower triangular, tri = 2: A^T (the
-// [d1, K] matrix) is lower triangular -- the stages that only multiply zeros are skipped.  chain_rows > 0 (one
-// segment, a multiple of 64): rows per accumulation chain of the tensor core; chains are added with rounded fp32
-// additions, in one launch by the pair kernel and by one launch per chain on the output otherwise.
+// [d1, K] matrix) is lower triangular -- the stages that only multiply zeros are skipped.  chain_rows > 0 (a
+// multiple of 64): rows per accumulation chain of the tensor core; chains are added with rounded fp32
+// additions, in one launch by the pair kernel and by one launch per chain on the output otherwise.  With several
+// segments a chain may run across their borders; only the pair kernel splits them.
 int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A, int64_t lda, int64_t a_rows,
                   int64_t a_x0, const void* B, int64_t ldb, int64_t b_rows, int64_t b_x0, bool symmetric, bool mirror,
                   int n_seg, int64_t seg_rows, const int* a_seg_y, const int* b_seg_y, float alpha, float beta,
@@ -627,13 +641,8 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
   if (d1 <= 0 || d2 <= 0 || seg_rows <= 0) return FPQ_OK;
   HessParams p{};
   p.d1 = d1; p.d2 = d2; p.ldc = ldc;
-  // no triangular skipping, enough 256-row tiles to fill the GPU: the 256 x 256 shape on CTA pairs (measured
-  // with the threshold at 64, 24 and 8 stages of K: the d = 14336 Cholesky-inverse chain 25.7, 25.0, 24.9 ms)
-  const int64_t total_stages = (int64_t)n_seg * ((seg_rows + BK - 1) / BK);
-  const int64_t rows256 = (d1 + 255) / 256, cols256 = (d2 + TILE_N - 1) / TILE_N;
-  const int64_t big_tiles = symmetric ? rows256 * (rows256 + 1) / 2 : rows256 * cols256;
-  const bool big = tri == 0 && total_stages >= 8 && big_tiles >= sm_count() / 2 && sm_count() >= 2;
-  if (!big && chain_rows > 0 && seg_rows > chain_rows) {
+  const bool big = gemm_atb_on_pairs(d1, d2, symmetric, n_seg, seg_rows);
+  if (!big && chain_rows > 0 && n_seg == 1 && seg_rows > chain_rows) {
     for (int64_t t0 = 0; t0 < seg_rows; t0 += chain_rows) {
       const int64_t n = seg_rows - t0 < chain_rows ? seg_rows - t0 : chain_rows;
       const int ya = (a_seg_y ? a_seg_y[0] : 0) + (int)t0, yb = (b_seg_y ? b_seg_y[0] : 0) + (int)t0;
