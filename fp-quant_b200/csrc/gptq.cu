@@ -22,6 +22,7 @@ int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A
                   int64_t a_x0, const void* B, int64_t ldb, int64_t b_rows, int64_t b_x0, bool symmetric, bool mirror,
                   int n_seg, int64_t seg_rows, const int* a_seg_y, const int* b_seg_y, float alpha, float beta,
                   int32_t* error_flag, cudaStream_t stream, int tri = 0, int64_t chain_rows = 0);
+bool gemm_atb_on_pairs(int64_t d1, int64_t d2, bool symmetric, int n_seg, int64_t seg_rows);
 }  // namespace fpq
 
 namespace fpq {
@@ -617,7 +618,7 @@ template <int G>
 __global__ void __launch_bounds__(G == 1 ? 256 : 512) gptq_block_kernel(float* __restrict__ W, int64_t rows, int64_t C,
                                                                         int64_t c1, const float* __restrict__ scales,
                                                                         const float* __restrict__ U,
-                                                                        __nv_bfloat16* __restrict__ ErrT3, int64_t lda,
+                                                                        __nv_bfloat16* __restrict__ ErrT3, int64_t lda, int64_t plane,
                                                                         uint8_t* __restrict__ codes,
                                                                         const int32_t* __restrict__ gidx, int n_groups) {
   extern __shared__ float Us[];   // NB rows of US_LD floats, then the reciprocals of the diagonal
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(G == 1 ? 256 : 512) gptq_block_kernel(float* _
     }
   }
   // The block's errors leave as the operand of the trailing update: three bf16 terms per value, transposed
-  // ([3 * 128, lda], plane p of column c at row p * 128 + c).  They are staged in shared memory (the image
+  // (plane p of column c is row c of the block, `plane` elements apart).  They are staged in shared memory (the image
   // of U is no longer needed) so that the global stores run along the rows.
   const int rb = (int)(blockDim.x >> 2);            // rows of this block
   const int es_ld = rb + 1;
@@ -723,8 +724,8 @@ __global__ void __launch_bounds__(G == 1 ? 256 : 512) gptq_block_kernel(float* _
       split3(v1, h1, m1, l1);
       __nv_bfloat16* dst = ErrT3 + (int64_t)c * lda + g;
       *reinterpret_cast<__nv_bfloat162*>(dst) = __halves2bfloat162(h0, h1);
-      *reinterpret_cast<__nv_bfloat162*>(dst + (int64_t)NB * lda) = __halves2bfloat162(m0, m1);
-      *reinterpret_cast<__nv_bfloat162*>(dst + (int64_t)2 * NB * lda) = __halves2bfloat162(l0, l1);
+      *reinterpret_cast<__nv_bfloat162*>(dst + plane) = __halves2bfloat162(m0, m1);
+      *reinterpret_cast<__nv_bfloat162*>(dst + 2 * plane) = __halves2bfloat162(l0, l1);
     }
   }
   if (!live) return;
@@ -951,12 +952,13 @@ extern "C" int fpq_cholesky_inverse_upper(const float* H, float* U, int64_t d, f
 
 namespace {
 int64_t align256(int64_t x) { return (x + 255) & ~(int64_t)255; }
+constexpr int64_t GPTQ_OB = 4;      // column blocks whose errors are applied to the rest of the weight together
 int64_t gptq_lda(int64_t rows) { return (rows + 63) & ~(int64_t)63; }
 }  // namespace
 
 extern "C" int64_t fpq_gptq_workspace_bytes(int64_t rows, int64_t cols) {
   if (rows <= 0 || cols <= 0) return 0;
-  return align256(rows * NB * (int64_t)sizeof(float)) + align256(3 * NB * gptq_lda(rows) * 2) + align256(3 * cols * cols * 2);
+  return align256(3 * GPTQ_OB * NB * gptq_lda(rows) * 2) + align256(3 * cols * cols * 2);
 }
 
 extern "C" int fpq_gptq_quantize(float* W, int64_t rows, int64_t cols, const float* scales, int group,
@@ -985,11 +987,11 @@ extern "C" int fpq_gptq_quantize_ordered(float* W, int64_t rows, int64_t cols, c
     FPQ_CHECK_CUDA(cudaFuncSetAttribute(gptq_block_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured[dev] = true;
   }
-  // workspace: (unused fp32 slab, kept so that the size helper does not change) | transposed three-term bf16 split of a block's errors | three-term bf16 split of U
-  const int64_t lda = gptq_lda(rows);
+  // workspace: transposed three-term bf16 split of the errors of GPTQ_OB blocks | three-term bf16 split of U
+  const int64_t lda = gptq_lda(rows), err_rows = GPTQ_OB * NB, plane = err_rows * lda;
   uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
-  __nv_bfloat16* errT3 = reinterpret_cast<__nv_bfloat16*>(ws + align256(rows * NB * (int64_t)sizeof(float)));
-  __nv_bfloat16* U3 = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(errT3) + align256(3 * NB * lda * 2));
+  __nv_bfloat16* errT3 = reinterpret_cast<__nv_bfloat16*>(ws);
+  __nv_bfloat16* U3 = reinterpret_cast<__nv_bfloat16*>(ws + align256(3 * plane * 2));
   if (cols > NB) {
     split3_rows_kernel<<<grid1d(cols * cols), 256, 0, st>>>(U, cols, cols, cols, U3, cols);
     FPQ_CHECK_LAUNCH();
@@ -1009,25 +1011,43 @@ extern "C" int fpq_gptq_quantize_ordered(float* W, int64_t rows, int64_t cols, c
   wpb = wpb < 4 ? 4 : (wpb > wpb_max ? wpb_max : wpb);
   const unsigned threads = (unsigned)wpb * 32;
   const unsigned grid = (unsigned)((units + wpb - 1) / wpb);
-  for (int64_t c1 = 0; c1 < cols; c1 += NB) {
-    const int n_groups = (int)(cols / group);
-    if (group_index)
-      gptq_block_kernel<1><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, errT3, lda, codes, group_index, n_groups);
-    else if (group == 16)
-      gptq_block_kernel<16><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, errT3, lda, codes, nullptr, n_groups);
-    else
-      gptq_block_kernel<32><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, errT3, lda, codes, nullptr, n_groups);
-    FPQ_CHECK_LAUNCH();
-    const int64_t c2 = c1 + NB;
-    if (c2 >= cols) break;
+  // The columns right of a block are updated in two levels: after a block only those of its group of GPTQ_OB blocks,
+  // after a group all others with the errors of the whole group.  The rest of W is then read and written once per
+  // group (it bounds the update of a single block: 128 columns of errors are 768 of K), and the accumulation chains in
+  // the tensor core stay as long as they were: 768, added with rounded fp32 additions.  Where the group's product is
+  // too small for the pair kernel, which splits chains, its blocks are applied one by one.
+  // Updates of a 14336 x 4096 loop 1.5 ms instead of 2.3 ms, of a 4096 x 14336 one 5.5 instead of 8.3.
+  const auto update = [&](int64_t e0, int64_t n_rows, int64_t u0, int64_t col, int64_t n) -> int {
     int a_y[6], b_y[6];
     for (int t = 0; t < 6; ++t) {
-      a_y[t] = pa[t] * NB;
-      b_y[t] = (int)(pb[t] * cols + c1);
+      a_y[t] = (int)(pa[t] * err_rows + e0);
+      b_y[t] = (int)(pb[t] * cols + u0);
     }
-    if (int rc = gemm_atb_bf16(W + c2, cols, rows, cols - c2, errT3, lda, 3 * NB, 0, U3, cols, 3 * cols, c2, false, false, 6,
-                               NB, a_y, b_y, -1.0f, 1.0f, error_flag, st))
-      return rc;
+    return gemm_atb_bf16(W + col, cols, rows, n, errT3, lda, 3 * err_rows, 0, U3, cols, 3 * cols, col, false, false, 6, n_rows,
+                         a_y, b_y, -1.0f, 1.0f, error_flag, st, 0, 6 * NB);
+  };
+  const int n_groups = (int)(cols / group);
+  for (int64_t g1 = 0; g1 < cols; g1 += err_rows) {
+    const int64_t g2 = g1 + err_rows < cols ? g1 + err_rows : cols;
+    for (int64_t c1 = g1; c1 < g2; c1 += NB) {
+      __nv_bfloat16* err = errT3 + (c1 - g1) * lda;
+      if (group_index)
+        gptq_block_kernel<1><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, err, lda, plane, codes, group_index, n_groups);
+      else if (group == 16)
+        gptq_block_kernel<16><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, err, lda, plane, codes, nullptr, n_groups);
+      else
+        gptq_block_kernel<32><<<grid, threads, smem, st>>>(W, rows, cols, c1, scales, U, err, lda, plane, codes, nullptr, n_groups);
+      FPQ_CHECK_LAUNCH();
+      if (c1 + NB < g2)
+        if (int rc = update(c1 - g1, NB, c1, c1 + NB, g2 - (c1 + NB))) return rc;
+    }
+    if (g2 >= cols) break;
+    if (gemm_atb_on_pairs(rows, cols - g2, false, 6, g2 - g1)) {
+      if (int rc = update(0, g2 - g1, g1, g2, cols - g2)) return rc;
+    } else {
+      for (int64_t c1 = g1; c1 < g2; c1 += NB)
+        if (int rc = update(c1 - g1, NB, c1, g2, cols - g2)) return rc;
+    }
   }
   return FPQ_OK;
 }
