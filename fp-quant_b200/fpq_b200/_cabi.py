@@ -63,6 +63,8 @@ _SIGNATURES = {
     "fpq_quantize_mxfp8_square": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "fpq_mxfp4_transpose_mxfp8": [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int, c_void_p],
     "fpq_mxfp4_transpose_dequant": [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_void_p],
+    "fpq_multiply_scales": [c_void_p, c_int, c_int64, c_void_p, c_int, c_void_p, c_void_p],
+    "fpq_group_scales": [c_void_p, c_int, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p],
     "fpq_linear_workspace_bytes": [c_int64, c_int64, c_int],
     "fpq_linear_forward": [c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
                            c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p],

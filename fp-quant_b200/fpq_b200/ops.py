@@ -249,6 +249,29 @@ def apply_scales(x: torch.Tensor, scales: torch.Tensor, group: int, out_kind: in
     return out
 
 
+def multiply_scales(q: torch.Tensor, scales: torch.Tensor, group: int) -> torch.Tensor:
+    """q * scales, one scale per `group` consecutive elements; contiguous q and scales of one dtype (bf16 or fp32)."""
+    out = torch.empty_like(q)
+    with _guard(q.device):
+        C.call("fpq_multiply_scales", q.data_ptr(), _dt(q), q.numel(), scales.data_ptr(), group, out.data_ptr(), _stream(q))
+    return out
+
+
+def group_scales(x: torch.Tensor, fmt: str, global_scale: Optional[torch.Tensor], nan_flag: torch.Tensor) -> torch.Tensor:
+    """fp32 [rows, cols/g]: the min-max scales of `quantize` without its other outputs; nan_flag (int32 [1] on x's device)
+    becomes 1 when one of them is NaN."""
+    x, rows, cols = _2d(x)
+    sf = torch.empty(rows, cols // GROUP_OF[fmt], dtype=torch.float32, device=x.device)
+    if fmt == "nvfp4":
+        if global_scale is None:
+            raise ValueError("nvfp4 needs a global_scale tensor")
+        global_scale = _cuda(global_scale, "global_scale").to(torch.float32)
+    with _guard(x.device):
+        C.call("fpq_group_scales", x.data_ptr(), _dt(x), rows, cols, FORMATS[fmt], _ptr(global_scale) if fmt == "nvfp4" else None,
+               sf.data_ptr(), nan_flag.data_ptr(), _stream(x))
+    return sf
+
+
 def pack_grid(q: torch.Tensor) -> torch.Tensor:
     q, rows, cols = _2d(q)
     out = torch.empty(rows, cols // 2, dtype=torch.uint8, device=q.device)

@@ -75,28 +75,27 @@ class Quantizer:
         parameters only matter for the MSE observer (quantizer.py:117-134)."""
         fmt = self._kernel_format
         gs = None
+        flags = torch.zeros(3, dtype=torch.int32, device=x.device)     # bits of max|x|, tensor scale bad, a scale is NaN
         if fmt == "nvfp4":
             gs = self._device_global_scale(x.device)
             if self._track_global_scale:
-                bits = ops.absmax_bits(x, 0)
-                status = torch.zeros(1, dtype=torch.int32, device=x.device)
-                ops.global_scale_update(bits, gs, status)
-                bad = (status != 0) | ~torch.isfinite(gs)
-                if self.deferred_checks is not None:
-                    self.deferred_checks.append(bad.reshape(()))
-                elif bool(bad.item()):
-                    raise ValueError(f"Global scale is not finite: {gs}")
+                ops.global_scale_update(ops.absmax_bits(x, 0, out=flags[0:1]), gs, flags[1:2])
         if self.observer == QuantizationObserver.MSE:
             scales = ops.mse_scales(x, fmt, gs, scale_search_iters, max_scale_shrink_factor, error_norm)
+            flags[2:3] = scales.isnan().any()
         else:
-            _, _, scales = ops.quantize(x, fmt, 0, gs, codes=False, scale_bytes=False, scales_f32=True)
+            scales = ops.group_scales(x, fmt, gs, flags[2:3])
         scales = scales.view(*x.shape[:-1], x.shape[-1] // self.group_size).to(x.dtype)
-        bad = scales.isnan().any()
+        zeros = torch.zeros_like(scales)
         if self.deferred_checks is not None:
-            self.deferred_checks.append(bad)
-        elif bool(bad.item()):
-            raise ValueError("Scales are not finite.")
-        return scales, torch.zeros_like(scales)
+            self.deferred_checks.append(flags[1:].any())
+        else:
+            _, bad_scale, bad_group = flags.tolist()                   # the only synchronisation, after everything is queued
+            if bad_scale:
+                raise ValueError(f"Global scale is not finite: {gs}")
+            if bad_group:
+                raise ValueError("Scales are not finite.")
+        return scales, zeros
 
     def raise_deferred_checks(self) -> None:
         """One synchronisation for all checks collected since `deferred_checks` was set to a list."""
@@ -122,6 +121,11 @@ class Quantizer:
     @torch.no_grad()
     def dequantize(self, q: torch.Tensor, scales: torch.Tensor, zeros: Optional[torch.Tensor] = None) -> torch.Tensor:
         s = scales.to(q.dtype)
+        if self.group_size and q.is_cuda and s.device == q.device and q.dtype in (torch.float32, torch.bfloat16) \
+                and q.dim() > 0 and s.shape == q.shape[:-1] + (q.shape[-1] // self.group_size,) \
+                and q.shape[-1] % self.group_size == 0 and type(q) is torch.Tensor and type(s) is torch.Tensor \
+                and q.is_contiguous() and s.is_contiguous() and q.data_ptr() % 16 == 0 and q.numel() > 0:
+            return ops.multiply_scales(q, s, self.group_size)
         if self.group_size:
             return (q.reshape(*q.shape[:-1], -1, self.group_size) * s.unsqueeze(-1)).reshape(q.shape)
         return q * s

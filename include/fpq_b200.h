@@ -285,6 +285,21 @@ int fpq_mxfp4_requantize_transposed(const uint8_t* codes_in, const uint8_t* scal
                                     uint8_t* codes, uint8_t* scale_bytes, int scale_layout, fpq_stream_t stream);
 
 /*
+ * out = q * (scale of its group) for n contiguous elements, q, scales and out of one dtype (Quantizer.dequantize,
+ * src/quantization/quantizer.py:170-181).  group: a multiple of 8 that divides n.
+ */
+int fpq_multiply_scales(const void* q, int dtype, int64_t n, const void* scales, int group, void* out,
+                        fpq_stream_t stream);
+
+/*
+ * The fp32 group scales of fpq_quantize alone (Quantizer.get_quantization_params, src/quantization/quantizer.py:107-168,
+ * min-max observer, no rotation): scales_f32 [rows, cols / g].  *nan_flag (optional) is set to 1 when one is NaN and left
+ * alone otherwise.
+ */
+int fpq_group_scales(const void* x, int dtype, int64_t rows, int64_t cols, int format, const float* global_scale,
+                     float* scales_f32, int32_t* nan_flag, fpq_stream_t stream);
+
+/*
  * The forward pass of a quantised linear layer in one call (FPQuant4x16NoMasterFn.forward,
  * inference_lib/src/fp_quant/module/linear_fns.py:484-528): fpq_quantize (or fpq_quantize_quest, or with up_bf16
  * fpq_quantize_silu_mul of gate = x) into `workspace`, then fpq_gemm_fp4.  x, up: bf16 [M, K]; out: bf16 [M, N].
