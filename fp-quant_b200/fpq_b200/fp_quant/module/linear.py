@@ -63,7 +63,7 @@ class FPQuantLinear(nn.Module):
         self.register_buffer("backward_hadamard_matrix", torch.empty(hg, hg, **kw))
         self._scales_blocked = None
         self._scales_blocked_key = None
-        self._constants = None
+        self._constants = {}
         self._constants_of = None
 
     # ------------------------------------------------------------------ load-time step
@@ -126,15 +126,26 @@ class FPQuantLinear(nn.Module):
         return self._scales_blocked
 
     def _gemm_constants(self) -> GemmConstants:
-        """What the passes derive from the two tensor scales, recomputed only when one of them changed (up to nine small
-        kernels per training step otherwise).  The tensors it was made from are kept and compared as objects, so an
-        address that is used again cannot pass for them."""
+        """What the passes derive from the two tensor scales, remade only when one of them changed (up to nine small kernels
+        per training step otherwise).  The tensors it was made from are kept and compared as objects, so an address that is
+        used again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written
+        yet; a stream that is being captured takes the set of an earlier pass (a capture starts after a synchronisation),
+        and keeps none of its own, whose values would only exist after a replay."""
         w, a = self.weight_global_scale, self.act_global_scale
         of = self._constants_of
         if of is None or of[0] is not w or of[1] is not a or of[2:] != (w._version, a._version, w.data_ptr(), a.data_ptr()):
-            self._constants = GemmConstants.make(w, a)
+            self._constants = {}
             self._constants_of = (w, a, w._version, a._version, w.data_ptr(), a.data_ptr())
-        return self._constants
+        stream = torch._C._cuda_getCurrentRawStream(w.device.index) if w.is_cuda else 0
+        kept = self._constants
+        consts = kept.get(stream)
+        if consts is None:
+            if w.is_cuda and torch.cuda.is_current_stream_capturing():
+                return next(iter(kept.values()), None) or GemmConstants(w, a)
+            if len(kept) >= 8:
+                kept = self._constants = {}
+            consts = kept[stream] = GemmConstants(w, a)
+        return consts
 
     def _gemm_alpha(self) -> torch.Tensor:
         """1 / (weight_global_scale * act_global_scale) as fp32 [1]."""

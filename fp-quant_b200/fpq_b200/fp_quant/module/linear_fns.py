@@ -6,7 +6,7 @@ weights raises like the reference does.  `FPQuant4x4MasterFn` runs both gradient
 """
 from __future__ import annotations
 
-from typing import NamedTuple, Optional, Tuple
+from typing import Optional, Tuple
 
 import torch
 from torch.autograd import Function
@@ -28,19 +28,26 @@ def plain_eager(x: torch.Tensor) -> bool:
             and torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None)
 
 
-class GemmConstants(NamedTuple):
-    """fp32 [1] tensors that follow from the two tensor scales."""
-    alpha: torch.Tensor          # `gemm_alpha`
-    act_scale: torch.Tensor
-    weight_scale: torch.Tensor
-    act_inverse: torch.Tensor    # 1 / act_scale
-    weight_inverse: torch.Tensor
+class GemmConstants:
+    """fp32 [1] tensors that follow from the two tensor scales: `alpha` (`gemm_alpha`), the scales themselves, and for the
+    MXFP8 backward their inverses, made when they are first asked for."""
 
-    @classmethod
     @torch.no_grad()
-    def make(cls, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor) -> "GemmConstants":
-        w, a = weight_global_scale.float().reshape(1), act_global_scale.float().reshape(1)
-        return cls(gemm_alpha(weight_global_scale, act_global_scale), a, w, 1.0 / a, 1.0 / w)
+    def __init__(self, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor):
+        self.alpha = gemm_alpha(weight_global_scale, act_global_scale)
+        self.weight_scale, self.act_scale = weight_global_scale.float().reshape(1), act_global_scale.float().reshape(1)
+        self._inverses = None
+
+    @torch.no_grad()
+    def inverses(self) -> Tuple[torch.Tensor, torch.Tensor]:
+        """(1 / act_scale, 1 / weight_scale).  Not kept when the stream is being captured: a graph's tensors hold nothing
+        before it is replayed."""
+        if self._inverses is not None:
+            return self._inverses
+        pair = (1.0 / self.act_scale, 1.0 / self.weight_scale)
+        if not torch.cuda.is_current_stream_capturing():
+            self._inverses = pair
+        return pair
 
 
 def forward_quantize(x: torch.Tensor, hadamard_matrix: torch.Tensor, global_scale: torch.Tensor,
@@ -189,7 +196,7 @@ def _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale,
     orientations, so the `nn` product is a `tn` product of the transposed copy.  `swizzled`: x_scales and w_scales
     already are in the layout the GEMM reads."""
     if constants is not None:
-        act_inverse, weight_inverse = constants.act_inverse, constants.weight_inverse
+        act_inverse, weight_inverse = constants.inverses()
     else:
         act_inverse, weight_inverse = ((1.0 / s.float()).reshape(1) for s in (act_global_scale, weight_global_scale))
 

@@ -346,10 +346,22 @@ def linear_forward(x: torch.Tensor, up: Optional[torch.Tensor], w_codes: torch.T
                    bias: Optional[torch.Tensor]) -> torch.Tensor:
     """quantise + `gemm_fp4` in one call: bf16 [.., N] of x bf16 [.., K] (times silu: `quantize_silu_mul(x, up)`).  The
     caller vouches for the types: contiguous bf16 x and up of one shape, w_codes u8 [N, K/2], swizzled weight scales,
-    fp32 [1] alpha (and global_scale for NVFP4), bf16 [N] bias or None, all on x's device."""
+    fp32 [1] alpha (and global_scale for NVFP4), bf16 [N] bias or None, all on x's device.
+    Long products take two calls instead: the host has time for them, and the output is allocated while the activations
+    are quantised (the first pass over 3001 x 5120 x 17408 25 us shorter, passes in a row 2 us).  The line lies where the
+    kernels take about as long as the host for two calls, 60 us."""
     n, k = w_codes.shape[0], x.shape[-1]
     m = x.numel() // k
     nv = fmt == "nvfp4"
+    if m * n * k > 150_000_000_000:
+        x2 = x.view(m, k)
+        if up is not None:
+            q, sb = quantize_silu_mul(x2, up.view(m, k), fmt, hadamard_group, global_scale)
+        elif quest:
+            q, sb, _ = quantize_quest(x2, hadamard_group, swizzled=True)
+        else:
+            q, sb, _ = quantize(x2, fmt, hadamard_group, global_scale if nv else None, swizzled=True)
+        return gemm_fp4(q, w_codes, sb, w_scales_swizzled, alpha, fmt, bias).view(x.shape[:-1] + (n,))
     sf_cols = k // 16 if nv else k // 32
     size = ((m * k // 2 + 255) & -256) + ((m + 127) & -128) * ((sf_cols + 3) & -4)
     dev = x.device

@@ -82,3 +82,37 @@ def test_training_matches_the_general_path(cuda_device, fmt, backward, method, g
         out.append((y, xi.grad, layer.weight.grad, layer.bias.grad))
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+def test_long_products_and_other_streams(cuda_device):
+    """Above the size where quantise and GEMM become two calls; passes on a stream of their own and from a graph that was
+    captured before any eager pass."""
+    k, n, m = 1024, 8192, 18000
+    for fmt, method, group in (("MXFP4", "quest", 32), ("NVFP4", "abs_max", 16)):
+        layer = _layer(cuda_device, k, n, fmt, method, group, torch.bfloat16)
+        x = torch.randn(m, k, device=cuda_device).bfloat16()
+        with torch.no_grad():
+            torch.cuda.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            layer._blocked_weight_scales()
+            from fpq_b200 import ops
+            ops.device_error_flag(cuda_device)
+            warm = _layer(cuda_device, k, n, fmt, method, group, torch.bfloat16)
+            warm(x), warm(x[:100])
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph):
+                captured = layer(x[:100])
+            got, small = layer(x), layer(x[:100])
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(captured, small) and torch.equal(got[:100], small)
+            side = torch.cuda.Stream()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                other = layer(x[:100])
+            side.synchronize()
+            assert torch.equal(other, small)
+            fused = layer._fused_forward
+            layer._fused_forward = lambda *a: None
+            assert torch.equal(layer(x), got)
+            layer._fused_forward = fused

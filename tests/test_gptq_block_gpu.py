@@ -1,0 +1,44 @@
+"""The column-block kernel where its variants meet: four to sixteen warps a block, safe and extreme divisors."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("group", [16, 32])
+@pytest.mark.parametrize("rows", [4737, 9473, 20001])     # five and nine warps a block, more than one block of sixteen per SM
+def test_rows_are_independent(cuda_device, rows, group):
+    """One block of columns (no trailing update): parts of up to 4096 rows give the same bits as all rows together.  Some
+    scales are so small or large that their warps take the IEEE divisions."""
+    from fpq_b200 import ops
+
+    g = torch.Generator(device=cuda_device).manual_seed(rows)
+    x = torch.randn(512, 128, device=cuda_device, generator=g)
+    H = x.t() @ x / 512
+    U, status = ops.cholesky_inverse_upper(H)
+    W = torch.randn(rows, 128, device=cuda_device, generator=g) * 0.02
+    s = torch.rand(rows, 128 // group, device=cuda_device, generator=g) * 0.01 + 0.004
+    s[5, 0], s[rows - 1, -1], s[4100] = 1e-33, 1e-35, 1e33
+    whole = W.clone()
+    codes = ops.gptq_quantize(whole, s, U, group)
+    for lo in range(0, rows, 4096):
+        part = W[lo:lo + 4096].clone()
+        want = ops.gptq_quantize(part, s[lo:lo + 4096].contiguous(), U, group)
+        assert torch.equal(codes[lo:lo + 4096], want) and torch.equal(whole[lo:lo + 4096], part)
+    ops.check_device_errors(cuda_device)
+
+
+def test_extreme_pivot_takes_the_general_division(cuda_device):
+    """A factor whose diagonal leaves the range of the reciprocal form against the same factor a power of two smaller: the
+    errors shrink exactly as the factor grows, so codes and weights agree."""
+    from fpq_b200 import ops
+
+    g = torch.Generator(device=cuda_device).manual_seed(0)
+    U = torch.triu(torch.randn(128, 128, device=cuda_device, generator=g) * 0.05)
+    U.diagonal().fill_(1.0)
+    W = torch.randn(64, 128, device=cuda_device, generator=g)
+    s = torch.rand(64, 8, device=cuda_device, generator=g) * 0.5 + 0.25
+    a, b = W.clone(), W.clone()
+    want = ops.gptq_quantize(a, s, U, 16)
+    got = ops.gptq_quantize(b, s, U * 2.0 ** 101, 16)       # err / 2^101, times 2^101 U
+    assert torch.equal(want, got) and torch.equal(a, b)
