@@ -342,7 +342,7 @@ int fpq_sgemm(const float* A, int64_t lda, const float* B, int64_t ldb, int b_tr
  * mirrored, as accumulate_hessian does (src/quantization/accumulate_hessian.py:20-148); alpha and beta
  * carry the running-mean factors of GPTQ.update (src/quantization/gptq.py:94-102), so the input is
  * not rescaled.  xa, xb: bf16 [tokens, d] row-major, d % 8 == 0.  error_flag as in fpq_gemm_fp4.
- * Tokens are processed in slabs of 4096 (one launch each) because the tensor core's accumulator truncates:
+ * Tokens are accumulated in chains of 4096, joined by rounded additions, because the tensor core's accumulator truncates:
  * 4.5e-6 relative Frobenius error against fp64 for any number of tokens.
  */
 int fpq_hessian_accumulate(float* H, int64_t d, const void* xa_bf16, const void* xb_bf16, int64_t tokens,
@@ -389,7 +389,7 @@ int64_t fpq_cholesky_workspace_floats(int64_t d);
  * U = upper-triangular factor with U^T U = H^-1: what `torch.linalg.cholesky(inv_sym(H), upper=True)`
  * returns (src/quantization/gptq.py:212-215, src/utils/linalg_utils.py:8-12), computed as one
  * Cholesky factorisation of the index-reversed H and one triangular inverse, all in fp32.
- * *status (device int32) becomes 1 when a pivot is not positive -- the reference then falls back to
+ * *status (device int32) becomes 1 when a pivot is not a positive normal number -- the reference then falls back to
  * the identity (gptq.py:216-217); the caller decides.  H is not modified; U must not alias H.
  * The large trailing updates and triangular-inverse products run on the tensor cores as three-term
  * bf16 splits (fp32-level accuracy); error_flag as for fpq_gemm_fp4.
