@@ -1191,7 +1191,11 @@ int launch_one(const QuantParams& params, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = use_dependent_launch() ? 1 : 0;
+  // Early launch is for short calls, where setting up counts.  Codes of an input that fills the chip more than once are
+  // launched in order: next to the tail of the previous layer's GEMM the early blocks cost more than they save (passes
+  // of 3001 x 5120 x 17408 in a row 149.7 us instead of 152.4; 8192 x 12288 x 4096 228 either way).
+  const bool early = MODE != MODE_CODES || blocks_needed <= (int64_t)sm_count() * per_sm;
+  cfg.numAttrs = early && use_dependent_launch() ? 1 : 0;
   FPQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, quant_kernel<GH, FMT, IN_BF16, MODE>, p));
   return FPQ_OK;
 }
