@@ -351,8 +351,9 @@ hessian_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 // committed to both, "accumulator empty" lives in the leader and collects the epilogue warps of both.
 //
 // A long K is walked in chains of `chain_stages` stages: each chain ends up in one of the two accumulators and is
-// added (rounded fp32 addition) to a running sum in the registers of the eight epilogue warps, 128 columns of one
-// row per thread, while the next chain's MMAs run.  The output is read and written once per tile.  Bound by the
+// added (rounded fp32 addition) to beta H in the registers of the eight epilogue warps, 128 columns of one row per
+// thread, while the next chain's MMAs run.  The output is read and written once per tile, and its bits are those of
+// one launch per chain, whichever kernel takes it: every element goes through the same additions.  Bound by the
 // tensor pipe, and by the power limit when it runs for long.  16384 tokens, one launch instead of one per 4096 tokens
 // with four epilogue warps and rows of tiles in order: d = 4096 197 us (1392 TFLOP/s) instead of 239, d = 14336
 // 2260 us (1490) instead of 2615; all of MR-GPTQ of a 4096 x 14336 linear over 262144 tokens 99.2 instead of 119.4 ms.
@@ -527,9 +528,27 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const int64_t i = (int64_t)rb * TILE + quarter * 32 + lane;
       const int64_t jbase = (int64_t)jblock * TILE;
       const bool active = jbase < p.d2 && !(p.symmetric && jblock > rb);   // not beyond the matrix / above the diagonal
-      float sum[TILE];
+      const bool live = active && i < p.d1;
+      float* hrow = p.H + i * p.ldc + jbase;
+      float v[TILE];                                         // beta H, then chain by chain + alpha acc
 #pragma unroll
-      for (int j = 0; j < TILE; ++j) sum[j] = 0.0f;
+      for (int c = 0; c < TILE / 32; ++c) {
+        const bool whole = jbase + (c + 1) * 32 <= p.d2 && p.vec8;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[c * 32 + j] = 0.0f;
+        if (live && p.beta != 0.0f) {
+          // a lane owns 128 contiguous bytes of its row: 32-byte accesses touch whole sectors
+          if (whole) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ld_global_f32x8(hrow + c * 32 + 8 * q, v + c * 32 + 8 * q);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (jbase + c * 32 + j < p.d2) v[c * 32 + j] = hrow[c * 32 + j];
+          }
+        }
+      }
+      float scale = p.beta;
       for (int k0 = 0; k0 < n_st && ok; k0 += p.chain_stages, ++chain_count) {
         const uint32_t buf = chain_count & 1, acc_parity = (chain_count >> 1) & 1;
         if (!mbar_wait_bounded(bar_acc_full + 8 * buf, acc_parity, abort_flag)) { ok = false; break; }
@@ -541,49 +560,34 @@ hessian_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             tc_ld_32x32b_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * TILE_N + half * TILE + c * 32, r);
             tc_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) v[c * 32 + j] = fmaf(scale, v[c * 32 + j], p.alpha * __uint_as_float(r[j]));
           }
         }
+        scale = 1.0f;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(lead_acc_empty + 8 * buf);
       }
       if (!ok) break;
-      if (active && i < p.d1) {
+      if (live) {
         const bool mirror = p.mirror && jblock < rb;
 #pragma unroll
         for (int c = 0; c < TILE / 32; ++c) {
           const int64_t j0 = jbase + c * 32;
-          float* hrow = p.H + i * p.ldc + j0;
-          float* v = sum + c * 32;
+          const float* vc = v + c * 32;
           if (j0 + 32 <= p.d2 && p.vec8) {
-            // a lane owns 128 contiguous bytes of its row: 32-byte accesses touch whole sectors
-            float h[32];
-            if (p.beta != 0.0f) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) ld_global_f32x8(hrow + 8 * q, h + 8 * q);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) h[j] = 0.0f;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = fmaf(p.beta, h[j], p.alpha * v[j]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) st_global_f32x8(hrow + 8 * q, v + 8 * q);
+            for (int q = 0; q < 4; ++q) st_global_f32x8(hrow + c * 32 + 8 * q, vc + 8 * q);
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (j0 + j < p.d2) {
-                v[j] = fmaf(p.beta, p.beta == 0.0f ? 0.0f : hrow[j], p.alpha * v[j]);
-                hrow[j] = v[j];
-              }
-            }
+            for (int j = 0; j < 32; ++j)
+              if (j0 + j < p.d2) hrow[c * 32 + j] = vc[j];
           }
           if (mirror) {
             // H[j, i]: consecutive lanes hold consecutive i, so each store instruction is coalesced
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (j0 + j < p.d2) p.H[(j0 + j) * p.ldc + i] = v[j];
+              if (j0 + j < p.d2) p.H[(j0 + j) * p.ldc + i] = vc[j];
           }
         }
       }
@@ -628,7 +632,7 @@ bool gemm_atb_on_pairs(int64_t d1, int64_t d2, bool symmetric, int n_seg, int64_
 // transposed.  tri = 1: B (as the [K, d2] matrix of one segment) is lower triangular, tri = 2: A^T (the
 // [d1, K] matrix) is lower triangular -- the stages that only multiply zeros are skipped.  chain_rows > 0 (a
 // multiple of 64): rows per accumulation chain of the tensor core; chains are added with rounded fp32
-// additions, in one launch by the pair kernel and by one launch per chain on the output otherwise.  With several
+// additions, in one launch by the pair kernel and by one launch per chain on the output otherwise (the same bits).  With several
 // segments a chain may run across their borders; only the pair kernel splits them.
 int gemm_atb_bf16(float* out, int64_t ldc, int64_t d1, int64_t d2, const void* A, int64_t lda, int64_t a_rows,
                   int64_t a_x0, const void* B, int64_t ldb, int64_t b_rows, int64_t b_x0, bool symmetric, bool mirror,

@@ -29,6 +29,24 @@ def test_chains_match_fp64(cuda_device, tokens, d):
     assert torch.equal(H, H.t())
 
 
+@pytest.mark.parametrize("tokens,d", [(4097, 3080), (8192 + 4032, 4104), (12288, 3072)])
+@pytest.mark.parametrize("beta", [0.0, 0.25])
+def test_one_update_is_chain_by_chain(cuda_device, tokens, d, beta):
+    """The bits of one update are those of its chains of 4096 tokens applied one after the other, each addition rounded into
+    the output: how far a run is split must not show in the Hessian."""
+    from fpq_b200 import ops
+
+    x = inputs.correlated_activations(tokens, d, seed=d).to(cuda_device)
+    h0 = torch.randn(d, d, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(d))
+    h0 = h0 + h0.t()
+    got, want = h0.clone(), h0.clone()
+    ops.hessian_accumulate(got, x, alpha=0.3, beta=beta)
+    for t in range(0, tokens, 4096):
+        ops.hessian_accumulate(want, x[t:t + 4096], alpha=0.3, beta=beta if t == 0 else 1.0)
+    ops.check_device_errors(cuda_device)
+    assert torch.equal(got, want)
+
+
 def test_output_rows_off_the_vector_alignment(cuda_device):
     """d = 3724: rows of 14896 bytes, not a multiple of 32; the trailing updates run on CTA pairs (big enough) and take
     the element-wise store.  fp32 chain: residual of U^T U H below 1e-3 for a Hessian of condition < 1e3."""
