@@ -102,22 +102,28 @@ __global__ void reflect_inplace_kernel(float* A, int64_t d) {
 
 // ------------------------------------------------------------------ diagonal block: factor + invert
 // One CTA factors the nb x nb (<= 128) diagonal block A (lower Cholesky, in place) and writes
-// L^-1 (lower) to Linv.  A non-positive or non-finite pivot sets *status and is replaced by 1 so
-// that the kernel always terminates with finite data.
+// L^-1 (lower; blocks right of the diagonal stay as the caller zeroed them) to Linv.  A non-positive or
+// non-finite pivot sets *status and is replaced by 1 so that the kernel always terminates.
+//
+// The arithmetic is right-looking elimination column by column, with c = A[:, k] and x = X[k, :] unscaled:
+//     A[i, j] = fma(-c_i, c_j / pivot, A[i, j])  (i, j > k),     X[i, :] = fma(-c_i, x / pivot, X[i, :])  (i > k),
+// 1 / pivot rounded, the columns of L and the rows of X divided by sqrt(pivot) at the end.  Every element goes through
+// these operations in the order of k whatever the blocking below, so the bits do not depend on it.
 //
 // The kernel is one chain of dependent steps, so it is laid out for a short chain: blocks of 32 columns in shared
 // memory.  A block's 32 x 32 diagonal part is factored by one warp, a row per lane, in registers; a step costs one
-// shuffle latency (the pivot and the whole column leave together, unscaled: A[i, j] -= c_i c_j / pivot), a reciprocal
-// and a fused multiply-add, no barrier.  Everything else is done by many threads at a time and meanwhile:
-//   phase 1   warp 0 factors D_p
-//   phase 2   warps 0-3: the rows below and D_p^-1   | warps 4-7: S_p = L_(p, <p) X_(<p)
-//             (one forward substitution per thread)  |
-//   phase 3   all: X_p = -D_p^-1 S_p, the trailing part -= L L^T
-// with X = L^-1 by blocks of rows.  128 x 128: 35 us; 48 us as one right-looking elimination with a barrier per column.
+// shuffle latency (the pivot and the whole column leave together), a reciprocal, a product and a fused multiply-add,
+// no barrier.  Everything else is done by many threads at a time:
+//   phase 1   warp 0 factors D_p                       | four warps: S_p = -C_(p, <p) X_(<p)
+//   phase 2   four warps, one vector a thread: the rows of C below D_p and the columns of X_p (from S_p, and from the
+//             unit vectors), by forward substitution
+//   phase 3   all: the trailing part -= C (C / pivot)^T
+// with C the unscaled columns of L and X = L^-1 by blocks of rows.
 constexpr int CD_LD = NB + 4;         // row stride in shared memory: 16-byte rows whose starts walk through the banks
 constexpr int CD_B = 32;              // block of columns
 constexpr int CD_SLD = 96 + 4;
-constexpr int CD_SMEM = (2 * NB * CD_LD + CD_B * CD_SLD + NB) * (int)sizeof(float);
+constexpr int CD_TLD = CD_B + 4;
+constexpr int CD_SMEM = (2 * NB * CD_LD + CD_B * CD_SLD + (96 + 2 * CD_B) * CD_TLD + NB + CD_B) * (int)sizeof(float);
 
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   unsigned long long r;
@@ -128,8 +134,9 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return *reinterpret_cast<float2*>(&r);
 }
 
-// Factor the 32 x 32 block at D in place (lower part; the upper part becomes zero), 1 / L[k, k] to rd.
-__device__ __forceinline__ void factor32(float* D, float* rd, int lane, int32_t* status) {
+// Factor the 32 x 32 block at D: its unscaled columns C in place (lower part) and transposed to DT, C / pivot transposed
+// to TT, 1 / pivot to pinv, 1 / sqrt(pivot) to rinv.
+__device__ __forceinline__ void factor32(float* D, float* DT, float* TT, float* pinv, float* rinv, int lane, int32_t* status) {
   float a[CD_B];
 #pragma unroll
   for (int q = 0; q < CD_B / 4; ++q) {
@@ -137,125 +144,102 @@ __device__ __forceinline__ void factor32(float* D, float* rd, int lane, int32_t*
     a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
   }
   bool bad = false;
-  float mine = 1.0f;                                       // this row's pivot
+  float my_piv = 1.0f, my_pinv = 1.0f;                     // of this row
 #pragma unroll
   for (int k = 0; k < CD_B; ++k) {
     const float c = a[k];
     float piv = __shfl_sync(0xffffffffu, c, k);
-    const bool ok = piv >= 1.17549435e-38f && piv <= 3.40282347e38f;
+    const bool ok = piv > 0.0f && isfinite(piv);
     piv = ok ? piv : 1.0f;
     bad |= !ok;
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
-    const float t0 = c * r;
-    const float t = fmaf(t0, fmaf(-piv, r, 1.0f), t0);     // one Newton step: c / pivot with full fp32 accuracy
+    const float r = __frcp_rn(piv);
     // rows at or above k get values that nothing reads
 #pragma unroll
-    for (int j = k + 1; j < CD_B; ++j) a[j] = fmaf(-t, __shfl_sync(0xffffffffu, c, j), a[j]);
+    for (int j = k + 1; j < CD_B; ++j) a[j] = fmaf(-c, __shfl_sync(0xffffffffu, c, j) * r, a[j]);
     if (lane == k) {
-      mine = piv;
-      a[k] = piv;
+      my_piv = piv;
+      my_pinv = r;
     }
   }
-  // the square roots wait until here, off the chain: column k is divided by sqrt(pivot k)
-  float rinv = rsqrtf(mine);
-  rinv = rinv * fmaf(-0.5f * mine * rinv, rinv, 1.5f);
-#pragma unroll
-  for (int k = 0; k < CD_B; ++k) a[k] *= __shfl_sync(0xffffffffu, rinv, k);
+  // the square roots wait until here, off the chain
+  float ri = rsqrtf(my_piv);
+  ri = ri * fmaf(-0.5f * my_piv * ri, ri, 1.5f);           // one Newton step: full fp32 accuracy
   if (bad && lane == 0) atomicExch(status, 1);
-  rd[lane] = rinv;
-#pragma unroll
-  for (int q = 0; q < CD_B / 4; ++q) {
-    float4 v;
-    v.x = 4 * q <= lane ? a[4 * q] : 0.0f;
-    v.y = 4 * q + 1 <= lane ? a[4 * q + 1] : 0.0f;
-    v.z = 4 * q + 2 <= lane ? a[4 * q + 2] : 0.0f;
-    v.w = 4 * q + 3 <= lane ? a[4 * q + 3] : 0.0f;
-    *reinterpret_cast<float4*>(D + lane * CD_LD + 4 * q) = v;
-  }
-}
-
-// v <- L^-1 v for the 32 x 32 lower block at L (every thread a right-hand side of its own; L is read as a broadcast).
-__device__ __forceinline__ void solve32(const float* L, const float* rd, float (&v)[CD_B]) {
+  rinv[lane] = ri;
+  pinv[lane] = my_pinv;
 #pragma unroll
   for (int k = 0; k < CD_B; ++k) {
-    float s = v[k];
+    DT[k * CD_TLD + lane] = a[k];
+    TT[k * CD_TLD + lane] = a[k] * __shfl_sync(0xffffffffu, my_pinv, k);
+  }
+#pragma unroll
+  for (int q = 0; q < CD_B / 4; ++q)
+    *reinterpret_cast<float4*>(D + lane * CD_LD + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+}
+
+// Forward substitution, every thread a vector of its own: v[j] = fma(-L[j, k], z_k, v[j]) for k < j in order, with
+// z_k = v[k] (rows of A: L holds C / pivot) or v[k] / pivot (columns of X: L holds C).  L comes transposed, as broadcasts.
+__device__ __forceinline__ void solve32(const float* LT, const float* pinv, bool divide, float (&v)[CD_B]) {
+#pragma unroll
+  for (int k = 0; k < CD_B; ++k) {
+    const float z = divide ? v[k] * pinv[k] : v[k];
 #pragma unroll
     for (int q = 0; q < CD_B / 4; ++q) {
-      if (4 * q >= k) continue;
-      const float4 l = *reinterpret_cast<const float4*>(L + k * CD_LD + 4 * q);
-      s = fmaf(-l.x, v[4 * q], s);
-      if (4 * q + 1 < k) s = fmaf(-l.y, v[4 * q + 1], s);
-      if (4 * q + 2 < k) s = fmaf(-l.z, v[4 * q + 2], s);
-      if (4 * q + 3 < k) s = fmaf(-l.w, v[4 * q + 3], s);
+      if (4 * q + 3 <= k) continue;
+      const float4 l = *reinterpret_cast<const float4*>(LT + k * CD_TLD + 4 * q);
+      if (4 * q > k) v[4 * q] = fmaf(-l.x, z, v[4 * q]);
+      if (4 * q + 1 > k) v[4 * q + 1] = fmaf(-l.y, z, v[4 * q + 1]);
+      if (4 * q + 2 > k) v[4 * q + 2] = fmaf(-l.z, z, v[4 * q + 2]);
+      v[4 * q + 3] = fmaf(-l.w, z, v[4 * q + 3]);
     }
-    v[k] = s * rd[k];
   }
 }
 
-// A[r0 + i, r0 + j] -= sum_k P[i, k] P[j, k] over the T x T sixteenths below (and on) the diagonal; P = 32 columns.
-template <int T>
-__device__ __forceinline__ void trailing32(float* A, int r0, int c0, int ty, int tx) {
-  float2 acc[T][T];
+// A[r0 + i, r0 + j] = fma(-C[i, k], T[j, k], .), k = 0 .. 31 in order, over the sixteenths on and below the diagonal.
+template <int N>
+__device__ __forceinline__ void trailing32(float* A, const float* Tp, int r0, int c0, int ty, int tx) {
+  float acc[N][N];
 #pragma unroll
-  for (int r = 0; r < T; ++r)
+  for (int r = 0; r < N; ++r)
 #pragma unroll
-    for (int c = 0; c < T; ++c) acc[r][c] = make_float2(0.0f, 0.0f);
+    for (int c = 0; c <= r; ++c) acc[r][c] = A[(r0 + ty + 16 * r) * CD_LD + r0 + tx + 16 * c];
 #pragma unroll
   for (int q = 0; q < CD_B / 4; ++q) {
-    float4 pi[T], pj[T];
+    float4 ci[N], tj[N];
 #pragma unroll
-    for (int r = 0; r < T; ++r) {
-      pi[r] = *reinterpret_cast<const float4*>(A + (r0 + ty + 16 * r) * CD_LD + c0 + 4 * q);
-      pj[r] = *reinterpret_cast<const float4*>(A + (r0 + tx + 16 * r) * CD_LD + c0 + 4 * q);
+    for (int r = 0; r < N; ++r) {
+      ci[r] = *reinterpret_cast<const float4*>(A + (r0 + ty + 16 * r) * CD_LD + c0 + 4 * q);
+      tj[r] = *reinterpret_cast<const float4*>(Tp + (tx + 16 * r) * CD_TLD + 4 * q);
     }
 #pragma unroll
-    for (int r = 0; r < T; ++r)
+    for (int r = 0; r < N; ++r)
 #pragma unroll
       for (int c = 0; c <= r; ++c) {
-        acc[r][c] = fma2(make_float2(pi[r].x, pi[r].y), make_float2(pj[c].x, pj[c].y), acc[r][c]);
-        acc[r][c] = fma2(make_float2(pi[r].z, pi[r].w), make_float2(pj[c].z, pj[c].w), acc[r][c]);
+        acc[r][c] = fmaf(-ci[r].x, tj[c].x, acc[r][c]);
+        acc[r][c] = fmaf(-ci[r].y, tj[c].y, acc[r][c]);
+        acc[r][c] = fmaf(-ci[r].z, tj[c].z, acc[r][c]);
+        acc[r][c] = fmaf(-ci[r].w, tj[c].w, acc[r][c]);
       }
   }
 #pragma unroll
-  for (int r = 0; r < T; ++r)
+  for (int r = 0; r < N; ++r)
 #pragma unroll
-    for (int c = 0; c <= r; ++c) A[(r0 + ty + 16 * r) * CD_LD + r0 + tx + 16 * c] -= acc[r][c].x + acc[r][c].y;
-}
-
-// X rows [32 p, 32 p + 32), columns left of the diagonal block: -X_pp S.  Eight threads a row, four columns of every block.
-__device__ __forceinline__ void inverse_row(float* __restrict__ X, const float* __restrict__ S, int p, int tid) {
-  const int row = tid >> 3, col = (tid & 7) * 4;
-  const float* D = X + (32 * p + row) * CD_LD + 32 * p;
-  float2 d[CD_B / 2];
-#pragma unroll
-  for (int q = 0; q < CD_B / 4; ++q) {
-    const float4 v = *reinterpret_cast<const float4*>(D + 4 * q);
-    d[2 * q] = make_float2(-v.x, -v.y);
-    d[2 * q + 1] = make_float2(-v.z, -v.w);
-  }
-  for (int jb = 0; jb < p; ++jb) {
-    float2 lo = make_float2(0.0f, 0.0f), hi = lo;
-#pragma unroll
-    for (int k = 0; k < CD_B; ++k) {                       // D is zero beyond k = row
-      const float dk = (k & 1) ? d[k / 2].y : d[k / 2].x;
-      const float4 sv = *reinterpret_cast<const float4*>(S + k * CD_SLD + jb * CD_B + col);
-      lo = fma2(make_float2(dk, dk), make_float2(sv.x, sv.y), lo);
-      hi = fma2(make_float2(dk, dk), make_float2(sv.z, sv.w), hi);
-    }
-    *reinterpret_cast<float4*>(X + (32 * p + row) * CD_LD + jb * CD_B + col) = make_float4(lo.x, lo.y, hi.x, hi.y);
-  }
+    for (int c = 0; c <= r; ++c) A[(r0 + ty + 16 * r) * CD_LD + r0 + tx + 16 * c] = acc[r][c];
 }
 
 __global__ void __launch_bounds__(256, 1) chol_diag_kernel(float* A, int64_t lda, float* Linv, int64_t ldi, int nb,
                                                         int32_t* status) {
   extern __shared__ __align__(16) float cd_smem[];
-  float* As = cd_smem;
-  float* X = As + NB * CD_LD;
-  float* S = X + NB * CD_LD;
-  float* rd = S + CD_B * CD_SLD;
+  float* As = cd_smem;                       // unscaled columns of L once they are final
+  float* Y = As + NB * CD_LD;                // rows of X / pivot
+  float* S = Y + NB * CD_LD;
+  float* Tp = S + CD_B * CD_SLD;             // rows below the block: C / pivot
+  float* DT = Tp + 96 * CD_TLD;
+  float* TT = DT + CD_B * CD_TLD;
+  float* rinv = TT + CD_B * CD_TLD;
+  float* pinv = rinv + NB;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool vec = nb == NB && lda % 4 == 0 && ldi % 4 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)Linv & 15) == 0;
+  const bool vec = nb == NB && lda % 4 == 0 && ((uintptr_t)A & 15) == 0;
   for (int o = tid; o < NB * NB / 4; o += 256) {
     const int i = o / (NB / 4), j = (o % (NB / 4)) * 4;
     float v[4];
@@ -266,53 +250,25 @@ __global__ void __launch_bounds__(256, 1) chol_diag_kernel(float* A, int64_t lda
       for (int q = 0; q < 4; ++q) v[q] = (i < nb && j + q < nb) ? A[(int64_t)i * lda + j + q] : (i == j + q ? 1.0f : 0.0f);
     }
     *reinterpret_cast<float4*>(As + i * CD_LD + j) = *reinterpret_cast<float4*>(v);
-    *reinterpret_cast<float4*>(X + i * CD_LD + j) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   }
   __syncthreads();
 #pragma unroll 1
   for (int p = 0; p < NB / CD_B; ++p) {
     const int c0 = CD_B * p, below = NB - c0 - CD_B;
-    float* D = As + c0 * CD_LD + c0;
-    if (warp == 0) factor32(D, rd + c0, lane, status);
-    __syncthreads();
-    if (warp < 4) {
-      // right-hand sides: the rows below, then (last warp) the unit vectors, whose solutions are the columns of D^-1
-      const bool unit = warp == 3;
-      if (unit || tid < below) {
-        float v[CD_B];
-        float* row = As + (c0 + CD_B + tid) * CD_LD + c0;
-#pragma unroll
-        for (int q = 0; q < CD_B / 4; ++q) {
-          float4 w = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (!unit) w = *reinterpret_cast<const float4*>(row + 4 * q);
-          v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
-        }
-        if (unit) {
-#pragma unroll
-          for (int k = 0; k < CD_B; ++k) v[k] = lane == k ? 1.0f : 0.0f;
-        }
-        solve32(D, rd + c0, v);
-        if (unit) {
-#pragma unroll
-          for (int k = 0; k < CD_B; ++k) X[(c0 + k) * CD_LD + c0 + lane] = v[k];
-        } else {
-#pragma unroll
-          for (int q = 0; q < CD_B / 4; ++q)
-            *reinterpret_cast<float4*>(row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        }
-      }
-    } else if (p > 0) {
-      // S = L[c0 .. c0 + 31, 0 .. c0 - 1] X[0 .. c0 - 1, 0 .. c0 - 1], X lower triangular by blocks
-      const int t = tid - 128, r = t >> 2, cq = (t & 3) * 4;
-      const float* Lr = As + (c0 + r) * CD_LD;
+    if (warp == 0) {
+      factor32(As + c0 * CD_LD + c0, DT, TT, pinv, rinv + c0, lane, status);
+    } else if (p > 0 && (warp & 3) != 0 && warp < 6) {     // warps 1, 2, 3, 5: not on warp 0's scheduler
+      // S = -C[c0 .. c0 + 31, 0 .. c0 - 1] Y[0 .. c0 - 1, 0 .. c0 - 1], Y lower triangular by blocks, k in order
+      const int t = (warp < 4 ? warp - 1 : 3) * 32 + lane, r = t >> 2, cq = (t & 3) * 4;
+      const float* Cr = As + (c0 + r) * CD_LD;
       for (int jb = 0; jb < p; ++jb) {
         const int j = jb * CD_B + cq;                      // columns j .. j + 3 and j + 16 .. j + 19
         float2 s0 = make_float2(0.0f, 0.0f), s1 = s0, s2 = s0, s3 = s0;
 #pragma unroll 8
         for (int k = jb * CD_B; k < c0; ++k) {
-          const float2 l = make_float2(Lr[k], Lr[k]);
-          const float4 x0 = *reinterpret_cast<const float4*>(X + k * CD_LD + j);
-          const float4 x1 = *reinterpret_cast<const float4*>(X + k * CD_LD + j + 16);
+          const float2 l = make_float2(-Cr[k], -Cr[k]);
+          const float4 x0 = *reinterpret_cast<const float4*>(Y + k * CD_LD + j);
+          const float4 x1 = *reinterpret_cast<const float4*>(Y + k * CD_LD + j + 16);
           s0 = fma2(l, make_float2(x0.x, x0.y), s0);
           s1 = fma2(l, make_float2(x0.z, x0.w), s1);
           s2 = fma2(l, make_float2(x1.x, x1.y), s2);
@@ -323,36 +279,68 @@ __global__ void __launch_bounds__(256, 1) chol_diag_kernel(float* A, int64_t lda
       }
     }
     __syncthreads();
-    if (p > 0) inverse_row(X, S, p, tid);
-    if (p == 0) trailing32<6>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
-    if (p == 1) trailing32<4>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
-    if (p == 2) trailing32<2>(As, c0 + CD_B, c0, tid >> 4, tid & 15);
+    if (warp < 4) {
+      // 128 vectors whatever p: `below` rows of A, then the c0 + 32 columns of X that reach this block of rows
+      const bool is_x = tid >= below;
+      const int col = tid - below;
+      float v[CD_B];
+      float* row = As + (c0 + CD_B + tid) * CD_LD + c0;    // of A
+      if (!is_x) {
+#pragma unroll
+        for (int q = 0; q < CD_B / 4; ++q) {
+          const float4 w = *reinterpret_cast<const float4*>(row + 4 * q);
+          v[4 * q] = w.x; v[4 * q + 1] = w.y; v[4 * q + 2] = w.z; v[4 * q + 3] = w.w;
+        }
+      } else if (col < c0) {
+#pragma unroll
+        for (int k = 0; k < CD_B; ++k) v[k] = S[k * CD_SLD + col];
+      } else {
+#pragma unroll
+        for (int k = 0; k < CD_B; ++k) v[k] = col - c0 == k ? 1.0f : 0.0f;
+      }
+      solve32(is_x ? DT : TT, pinv, is_x, v);
+      if (!is_x) {
+        float* trow = Tp + tid * CD_TLD;
+#pragma unroll
+        for (int q = 0; q < CD_B / 4; ++q) {
+          *reinterpret_cast<float4*>(row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          const float4 r = *reinterpret_cast<const float4*>(pinv + 4 * q);
+          *reinterpret_cast<float4*>(trow + 4 * q) =
+              make_float4(v[4 * q] * r.x, v[4 * q + 1] * r.y, v[4 * q + 2] * r.z, v[4 * q + 3] * r.w);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < CD_B; ++k) {
+          Y[(c0 + k) * CD_LD + col] = v[k] * pinv[k];
+          if (c0 + k < nb && col < nb) Linv[(int64_t)(c0 + k) * ldi + col] = v[k] * rinv[c0 + k];
+        }
+      }
+    }
+    __syncthreads();
+    if (p == 0) trailing32<6>(As, Tp, c0 + CD_B, c0, tid >> 4, tid & 15);
+    if (p == 1) trailing32<4>(As, Tp, c0 + CD_B, c0, tid >> 4, tid & 15);
+    if (p == 2) trailing32<2>(As, Tp, c0 + CD_B, c0, tid >> 4, tid & 15);
     __syncthreads();
   }
   for (int o = tid; o < NB * NB / 4; o += 256) {
     const int i = o / (NB / 4), j = (o % (NB / 4)) * 4;
-    float a[4], x[4];
+    float a[4], r[4];
     *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(As + i * CD_LD + j);
-    *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(X + i * CD_LD + j);
+    *reinterpret_cast<float4*>(r) = *reinterpret_cast<const float4*>(rinv + j);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (j + q > i) a[q] = 0.0f;                          // above the diagonal: what the updates left there
+    for (int q = 0; q < 4; ++q) a[q] = j + q > i ? 0.0f : a[q] * r[q];   // above the diagonal: what the updates left there
     if (vec) {
       *reinterpret_cast<float4*>(A + (int64_t)i * lda + j) = *reinterpret_cast<float4*>(a);
-      *reinterpret_cast<float4*>(Linv + (int64_t)i * ldi + j) = *reinterpret_cast<float4*>(x);
     } else {
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (i < nb && j + q < nb) {
-          A[(int64_t)i * lda + j + q] = a[q];
-          Linv[(int64_t)i * ldi + j + q] = x[q];
-        }
+        if (i < nb && j + q < nb) A[(int64_t)i * lda + j + q] = a[q];
     }
   }
 }
 
 // ------------------------------------------------------------------ panel below a diagonal block
-// A[i, 0..127] <- sum_k A[i, k] Linv[j, k] (k <= j) in place for `rows` rows: L21 = A21 L11^-T.  A CTA takes 32 rows, so
+// A[i, 0..127] <- sum_k A[i, k] Linv[j, k] (k <= j, in order) in place for `rows` rows: L21 = A21 L11^-T.  A CTA takes 32 rows, so
 // that even a short panel spreads over the SMs, and holds Linv in shared memory; a thread has 2 x 8 outputs, the part
 // of Linv above its diagonal is skipped.  Latency-bound; as a 128 x 128-tile matrix product on at most 112 CTAs it took
 // 18 to 20 us a panel on average, here 10 (d = 4096) to 15 (d = 14336).
@@ -377,14 +365,14 @@ __global__ void __launch_bounds__(256, 2) chol_panel_kernel(float* A, int64_t ld
     *reinterpret_cast<float4*>((is_l ? Ls + i * CD_LD : Ps + (i - NB) * CD_LD) + j) = v;
   }
   __syncthreads();
-  float2 acc[2][8];
+  float acc[2][8];
 #pragma unroll
   for (int r = 0; r < 2; ++r)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[r][c] = make_float2(0.0f, 0.0f);
+    for (int c = 0; c < 8; ++c) acc[r][c] = 0.0f;
 #pragma unroll
   for (int kb = 0; kb < 8; ++kb) {                         // sixteen k at a time: columns tx + 16 c with c >= kb need them
-#pragma unroll
+#pragma unroll 2
     for (int q = 0; q < 4; ++q) {
       const int k = 16 * kb + 4 * q;
       const float4 a0 = *reinterpret_cast<const float4*>(Ps + ty * CD_LD + k);
@@ -392,10 +380,8 @@ __global__ void __launch_bounds__(256, 2) chol_panel_kernel(float* A, int64_t ld
 #pragma unroll
       for (int c = kb; c < 8; ++c) {
         const float4 l = *reinterpret_cast<const float4*>(Ls + (tx + 16 * c) * CD_LD + k);
-        acc[0][c] = fma2(make_float2(a0.x, a0.y), make_float2(l.x, l.y), acc[0][c]);
-        acc[0][c] = fma2(make_float2(a0.z, a0.w), make_float2(l.z, l.w), acc[0][c]);
-        acc[1][c] = fma2(make_float2(a1.x, a1.y), make_float2(l.x, l.y), acc[1][c]);
-        acc[1][c] = fma2(make_float2(a1.z, a1.w), make_float2(l.z, l.w), acc[1][c]);
+        acc[0][c] = fmaf(a0.w, l.w, fmaf(a0.z, l.z, fmaf(a0.y, l.y, fmaf(a0.x, l.x, acc[0][c]))));
+        acc[1][c] = fmaf(a1.w, l.w, fmaf(a1.z, l.z, fmaf(a1.y, l.y, fmaf(a1.x, l.x, acc[1][c]))));
       }
     }
   }
@@ -404,7 +390,7 @@ __global__ void __launch_bounds__(256, 2) chol_panel_kernel(float* A, int64_t ld
     const int64_t row = r0 + ty + 16 * r;
     if (row >= rows) continue;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) A[row * lda + tx + 16 * c] = acc[r][c].x + acc[r][c].y;
+    for (int c = 0; c < 8; ++c) A[row * lda + tx + 16 * c] = acc[r][c];
   }
 }
 

@@ -389,7 +389,7 @@ int64_t fpq_cholesky_workspace_floats(int64_t d);
  * U = upper-triangular factor with U^T U = H^-1: what `torch.linalg.cholesky(inv_sym(H), upper=True)`
  * returns (src/quantization/gptq.py:212-215, src/utils/linalg_utils.py:8-12), computed as one
  * Cholesky factorisation of the index-reversed H and one triangular inverse, all in fp32.
- * *status (device int32) becomes 1 when a pivot is not a positive normal number -- the reference then falls back to
+ * *status (device int32) becomes 1 when a pivot is not positive or not finite -- the reference then falls back to
  * the identity (gptq.py:216-217); the caller decides.  H is not modified; U must not alias H.
  * The large trailing updates and triangular-inverse products run on the tensor cores as three-term
  * bf16 splits (fp32-level accuracy); error_flag as for fpq_gemm_fp4.

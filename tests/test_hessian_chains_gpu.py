@@ -1,5 +1,6 @@
 """The accumulation chains and tile bands of the Hessian / A^T B kernel where they can go wrong: a chain of one token,
 ragged last chains, one to many bands, tiles beyond the matrix, an output whose rows are not 32-byte aligned."""
+import numpy as np
 import pytest
 import torch
 
@@ -88,3 +89,60 @@ def test_bad_pivots_are_reported(cuda_device):
         U, status = ops.cholesky_inverse_upper(H)
         assert int(status) == 1
     ops.check_device_errors(cuda_device)
+
+
+def _fma(a, b, c):
+    """fl32(a * b + c) of float32 arrays, rounded once: the product is exact in fp64, the sum is rounded to odd there."""
+    prod = a.astype(np.float64) * b.astype(np.float64)
+    c = c.astype(np.float64)
+    s = prod + c
+    t = s - prod
+    err = (prod - (s - t)) + (c - t)
+    bits = s.view(np.int64)
+    step = np.where((err > 0) == (s > 0), 1, -1)
+    return np.where((err != 0) & (bits & 1 == 0), bits + step, bits).view(np.float64).astype(np.float32)
+
+
+@pytest.mark.parametrize("d", [128, 100, 33, 1])
+def test_diagonal_block_is_right_looking_elimination(cuda_device, d):
+    """One block: bit for bit the elimination column by column, A[i, j] = fma(-c_i, c_j / pivot, .) and the same for the rows of
+    the inverse, whatever order the kernel works in (1 / sqrt(pivot) from the device's rsqrt and one Newton step)."""
+    from fpq_b200 import ops
+
+    x = torch.randn(2 * d + 8, d, generator=torch.Generator().manual_seed(d))
+    H = x.t() @ x / (2 * d)
+    H.diagonal().add_(0.05)
+    U, status = ops.cholesky_inverse_upper(H.to(cuda_device))
+    assert int(status) == 0
+    a = H.numpy()[::-1, ::-1].copy()
+    inv = np.eye(d, dtype=np.float32)
+    out = np.zeros((d, d), dtype=np.float32)
+    for k in range(d):
+        c, piv = a[:, k].copy(), a[k, k]
+        rec = np.float32(1) / piv
+        low = slice(k + 1, d)
+        a[low, low] = _fma(-c[low, None] + 0 * a[low, low], (c[low] * rec)[None, :] + 0 * a[low, low], a[low, low])
+        inv[low] = _fma(-c[low, None] + 0 * inv[low], (inv[k] * rec)[None, :] + 0 * inv[low], inv[low])
+        r = torch.rsqrt(torch.tensor([piv], device=cuda_device)).cpu().numpy()
+        r = r * _fma((np.float32(-0.5) * piv) * r, r, np.full(1, 1.5, np.float32))
+        out[k] = inv[k] * r[0]
+    assert np.array_equal(U.cpu().numpy()[::-1, ::-1], out)
+
+
+def test_largest_and_smallest_pivots(cuda_device):
+    """Pivots near the ends of fp32, whose reciprocals are subnormal or nearly overflow, are eliminated like any other."""
+    from fpq_b200 import ops
+
+    d = 200
+    for big, c in ((2e38, 2e19), (9e37, 1e19), (8e-39, 4e-20)):
+        for i in (150, 60):                          # in the first and the second block
+            H = 10 * torch.eye(d, dtype=torch.float64)
+            H[i, i] = big
+            H[i, 3] = H[3, i] = c                    # rows are eliminated from the last to the first
+            H = H.float()
+            low = torch.linalg.cholesky(H.double().flip(0, 1))
+            want = torch.linalg.solve_triangular(low, torch.eye(d, dtype=torch.float64), upper=False).flip(0, 1)
+            U, status = ops.cholesky_inverse_upper(H.to(cuda_device))
+            assert int(status) == 0
+            # 1 / 2e38 as a subnormal has 21 bits
+            assert torch.allclose(U.cpu().double(), want, rtol=2e-6, atol=0)
