@@ -1079,17 +1079,19 @@ extern "C" int fpq_gptq_quantize_ordered(float* W, int64_t rows, int64_t cols, c
   const unsigned grid = (unsigned)((units + wpb - 1) / wpb);
   // The columns right of a block are updated in two levels: after a block only those of its group of GPTQ_OB blocks,
   // after a group all others with the errors of the whole group.  The rest of W is then read and written once per
-  // group (it bounds the update of a single block: 128 columns of errors are 768 of K), and the accumulation chains in
-  // the tensor core stay as long as they were: 768, added with rounded fp32 additions.  Where the group's product is
-  // too small for the pair kernel, which splits chains, its blocks are applied one by one.
+  // group (it bounds the update of a single block: 128 columns of errors are 768 of K).  Every block keeps a chain of its
+  // own in the tensor core, subtracted from W by a rounded fp32 addition, in the order of the blocks: an element sees
+  // the same operations whether its group is one product or (where that is too small for the pair kernel, the one that
+  // splits chains) a product per block, so the codes of a row do not depend on the number of rows.
   // Updates of a 14336 x 4096 loop 1.5 ms instead of 2.3 ms, of a 4096 x 14336 one 5.5 instead of 8.3.
   const auto update = [&](int64_t e0, int64_t n_rows, int64_t u0, int64_t col, int64_t n) -> int {
-    int a_y[6], b_y[6];
-    for (int t = 0; t < 6; ++t) {
-      a_y[t] = (int)(pa[t] * err_rows + e0);
-      b_y[t] = (int)(pb[t] * cols + u0);
-    }
-    return gemm_atb_bf16(W + col, cols, rows, n, errT3, lda, 3 * err_rows, 0, U3, cols, 3 * cols, col, false, false, 6, n_rows,
+    int a_y[6 * GPTQ_OB], b_y[6 * GPTQ_OB], segs = 0;
+    for (int64_t r = 0; r < n_rows; r += NB)
+      for (int t = 0; t < 6; ++t, ++segs) {
+        a_y[segs] = (int)(pa[t] * err_rows + e0 + r);
+        b_y[segs] = (int)(pb[t] * cols + u0 + r);
+      }
+    return gemm_atb_bf16(W + col, cols, rows, n, errT3, lda, 3 * err_rows, 0, U3, cols, 3 * cols, col, false, false, segs, NB,
                          a_y, b_y, -1.0f, 1.0f, error_flag, st, 0, 6 * NB);
   };
   const int n_groups = (int)(cols / group);
@@ -1108,7 +1110,7 @@ extern "C" int fpq_gptq_quantize_ordered(float* W, int64_t rows, int64_t cols, c
         if (int rc = update(c1 - g1, NB, c1, c1 + NB, g2 - (c1 + NB))) return rc;
     }
     if (g2 >= cols) break;
-    if (gemm_atb_on_pairs(rows, cols - g2, false, 6, g2 - g1)) {
+    if (gemm_atb_on_pairs(rows, cols - g2, false, (int)(6 * ((g2 - g1) / NB)), NB)) {
       if (int rc = update(0, g2 - g1, g1, g2, cols - g2)) return rc;
     } else {
       for (int64_t c1 = g1; c1 < g2; c1 += NB)

@@ -49,7 +49,7 @@ struct Shape {
   static constexpr int DYN_BYTES = TOTAL + 1024;
 };
 
-constexpr int MAX_SEGMENTS = 6;
+constexpr int MAX_SEGMENTS = 24;     // six cross products of each of four column blocks
 
 struct HessParams {
   int64_t d1, d2, ldc;  // output rows (A's width), columns (B's width), row stride of the output

@@ -42,3 +42,30 @@ def test_extreme_pivot_takes_the_general_division(cuda_device):
     want = ops.gptq_quantize(a, s, U, 16)
     got = ops.gptq_quantize(b, s, U * 2.0 ** 101, 16)       # err / 2^101, times 2^101 U
     assert torch.equal(want, got) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("cols", [1408, 2048])        # a ragged last group of blocks, whole groups
+@pytest.mark.parametrize("group", [16, 32])
+def test_slabs_of_rows_give_the_bits_of_the_whole(cuda_device, cols, group):
+    """Many columns: the columns beyond a group are updated by one product where there are rows enough for the pair kernel, and
+    block by block elsewhere (all 9473 rows: pairs for every group; 6344 of them: the first groups; 3000 and fewer:
+    nowhere).  The codes and weights of a row must not depend on which."""
+    from fpq_b200 import ops
+
+    rows = 9473
+    g = torch.Generator(device=cuda_device).manual_seed(cols)
+    x = torch.randn(4 * cols, 32, device=cuda_device, generator=g) @ torch.randn(32, cols, device=cuda_device, generator=g) / 6
+    x += torch.randn(4 * cols, cols, device=cuda_device, generator=g)
+    H = x.t() @ x / (4 * cols)
+    H.diagonal().add_(0.01)
+    U, status = ops.cholesky_inverse_upper(H)
+    assert int(status) == 0
+    W = torch.randn(rows, cols, device=cuda_device, generator=g) * 0.02
+    s = W.view(rows, cols // group, group).abs().amax(-1) / 6
+    whole = W.clone()
+    codes = ops.gptq_quantize(whole, s, U, group)
+    for lo, hi in ((0, 3000), (3000, 3128), (3128, 3129), (3129, rows)):
+        part = W[lo:hi].clone()
+        want = ops.gptq_quantize(part, s[lo:hi].contiguous(), U, group)
+        assert torch.equal(codes[lo:hi], want) and torch.equal(whole[lo:hi], part)
+    ops.check_device_errors(cuda_device)
