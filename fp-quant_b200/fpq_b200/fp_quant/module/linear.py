@@ -13,7 +13,7 @@ from ... import ops
 from ...rotation import classify_rotation, sylvester
 from ..utils.config import FPQuantConfig, FPQuantDtype, validate_config
 from .linear_fns import (FPQuant4x4MasterFn, FPQuant4x8MasterFn, FPQuant4x8NoMasterFn, FPQuant4x16MasterFn, FPQuant4x16NoMasterFn,
-                         GemmConstants, _linear_forward, forward_gemm_blocked, forward_quantize, gemm_alpha, plain_eager)
+                         ConstantsCache, GemmConstants, _linear_forward, forward_gemm_blocked, forward_quantize, gemm_alpha, plain_eager)
 from .pseudoquant_linear_fns import PseudoQuant4x16MasterFn, PseudoQuant4x16NoMasterFn, forward_pseudoquantize
 from .qutlass_ops import (HAS_QUTLASS, fused_silu_mul_quantize_blocked_op,  # noqa: F401  (HAS_QUTLASS: API compatibility)
                           swizzle_scales_op)
@@ -63,8 +63,7 @@ class FPQuantLinear(nn.Module):
         self.register_buffer("backward_hadamard_matrix", torch.empty(hg, hg, **kw))
         self._scales_blocked = None
         self._scales_blocked_key = None
-        self._constants = {}
-        self._constants_of = None
+        self._constants = ConstantsCache()
 
     # ------------------------------------------------------------------ load-time step
     @torch.no_grad()
@@ -125,27 +124,12 @@ class FPQuantLinear(nn.Module):
             self._scales_blocked_key = key
         return self._scales_blocked
 
-    def _gemm_constants(self) -> GemmConstants:
-        """What the passes derive from the two tensor scales, remade only when one of them changed (up to nine small kernels
-        per training step otherwise).  The tensors it was made from are kept and compared as objects, so an address that is
-        used again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written
-        yet; a stream that is being captured takes the set of an earlier pass (a capture starts after a synchronisation),
-        and keeps none of its own, whose values would only exist after a replay."""
+    def _gemm_constants(self, training: bool = False) -> GemmConstants:
+        """What the passes derive from the two tensor scales (see `ConstantsCache`)."""
         w, a = self.weight_global_scale, self.act_global_scale
-        of = self._constants_of
-        if of is None or of[0] is not w or of[1] is not a or of[2:] != (w._version, a._version, w.data_ptr(), a.data_ptr()):
-            self._constants = {}
-            self._constants_of = (w, a, w._version, a._version, w.data_ptr(), a.data_ptr())
-        stream = torch._C._cuda_getCurrentRawStream(w.device.index) if w.is_cuda else 0
-        kept = self._constants
-        consts = kept.get(stream)
-        if consts is None:
-            if w.is_cuda and torch.cuda.is_current_stream_capturing():
-                return next(iter(kept.values()), None) or GemmConstants(w, a)
-            if len(kept) >= 8:
-                kept = self._constants = {}
-            consts = kept[stream] = GemmConstants(w, a)
-        return consts
+        if not w.is_cuda:
+            return self._constants.get(w, a, 0, False)
+        return self._constants.get(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing(), follow=training)
 
     def _gemm_alpha(self) -> torch.Tensor:
         """1 / (weight_global_scale * act_global_scale) as fp32 [1]."""
@@ -211,7 +195,7 @@ class FPQuantLinear(nn.Module):
 
     def _training_constants(self, x: torch.Tensor):
         """The cached constants for a training pass; None (they are derived on the way) under a tracer."""
-        return self._gemm_constants() if plain_eager(x) else None
+        return self._gemm_constants(training=True) if plain_eager(x) else None
 
     # ------------------------------------------------------------------ forward
     def forward(self, x) -> torch.Tensor:

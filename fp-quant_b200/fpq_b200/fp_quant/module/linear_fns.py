@@ -50,6 +50,42 @@ class GemmConstants:
         return pair
 
 
+class ConstantsCache:
+    """`GemmConstants` of one layer, remade only when one of its two tensor scales changed (up to nine small kernels per
+    training step otherwise).  The tensors a set was made from are kept and compared as objects, so an address that is used
+    again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written yet."""
+
+    def __init__(self):
+        self._of = None         # (key, {stream: set}), replaced as a whole: threads see one state or the other
+        self._captured = []     # sets whose addresses a CUDA graph holds: kept for as long as the layer lives
+
+    def get(self, w: torch.Tensor, a: torch.Tensor, stream: int, capturing: bool, follow: bool = False) -> GemmConstants:
+        """The set for a pass on `stream`.  While that stream is being captured: with `follow` a set of the graph's own, whose
+        replays follow the scales (training passes, whose scales may be updated in place); else the set of an earlier
+        pass, which costs the replays nothing, frozen as it is now.  Nothing made inside a capture is kept: its values
+        only exist after a replay."""
+        if capturing and follow:
+            return GemmConstants(w, a)
+        of = self._of
+        key = (w._version, a._version, w.data_ptr(), a.data_ptr())
+        if of is None or of[0] is not w or of[1] is not a or of[2] != key:
+            of = self._of = (w, a, key, {})
+        kept = of[3]
+        consts = kept.get(stream)
+        if not capturing:
+            if consts is None:
+                if len(kept) >= 8:
+                    kept.clear()
+                consts = kept[stream] = GemmConstants(w, a)
+            return consts
+        consts = consts or next(iter(kept.values()), None)
+        if consts is None:
+            return GemmConstants(w, a)
+        if not any(c is consts for c in self._captured):
+            self._captured.append(consts)
+        return consts
+
+
 def forward_quantize(x: torch.Tensor, hadamard_matrix: torch.Tensor, global_scale: torch.Tensor,
                      dtype: FPQuantDtype, forward_method: str) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor]]:
     """rotate + quantise -> (codes, row-major padded scales, mask) (linear_fns.py:27-50)."""

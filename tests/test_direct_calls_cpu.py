@@ -1,0 +1,69 @@
+"""What a layer keeps between passes."""
+import threading
+import weakref
+
+import torch
+
+from fpq_b200.fp_quant.module.linear_fns import ConstantsCache
+
+
+def _scales():
+    return torch.tensor([3.0], dtype=torch.bfloat16), torch.tensor([3.0], dtype=torch.bfloat16)
+
+
+def test_a_captured_graphs_constants_outlive_other_streams_and_new_scales():
+    """What a capture was given stays alive with the cache, whatever streams and scales come after."""
+    w, a = _scales()
+    cache = ConstantsCache()
+    own = cache.get(w, a, 1, False)
+    held = [weakref.ref(cache.get(w, a, 1, True)), weakref.ref(cache.get(w, a, 2, True))]     # its own stream's set, another's
+    assert held[0]() is own and held[1]() is own
+    kept = weakref.ref(cache.get(w, a, 3, False))
+    del own
+    for stream in range(4, 24):
+        assert cache.get(w, a, stream, False) is cache.get(w, a, stream, False)
+    w.mul_(2)
+    for stream in range(1, 24):
+        assert float(cache.get(w, a, stream, False).alpha) == float((1.0 / (w * a)).float())
+    assert all(r() is not None for r in held) and kept() is None
+    assert len(cache._of[3]) <= 8
+
+
+def test_what_a_capture_makes_is_not_kept():
+    w, a = _scales()
+    cache = ConstantsCache()
+    first = cache.get(w, a, 1, True)                       # no earlier pass: made inside the graph
+    assert cache.get(w, a, 1, False) is not first
+    eager = cache.get(w, a, 1, False)
+    follow = cache.get(w, a, 1, True, follow=True)         # a training step's graph derives its own
+    assert follow is not eager and cache.get(w, a, 1, False) is eager
+
+
+def test_constants_follow_the_scales():
+    w, a = _scales()
+    cache = ConstantsCache()
+    first = cache.get(w, a, 1, False)
+    assert cache.get(w, a, 1, False) is first
+    a.mul_(0.5)
+    second = cache.get(w, a, 1, False)
+    assert second is not first and float(second.act_scale) == 1.5
+    other = w.clone()
+    assert cache.get(other, a, 1, False) is not second     # another object, equal values
+    errors = []
+
+    def passes(scale):
+        try:
+            mine = torch.tensor([scale], dtype=torch.bfloat16)
+            for i in range(300):
+                got = cache.get(mine if i % 3 else other, a, i % 11, False)
+                if float(got.weight_scale) != (scale if i % 3 else 3.0):
+                    errors.append(i)
+        except Exception as e:                              # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=passes, args=(float(2 ** i),)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors

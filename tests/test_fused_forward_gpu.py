@@ -116,3 +116,63 @@ def test_long_products_and_other_streams(cuda_device):
             layer._fused_forward = lambda *a: None
             assert torch.equal(layer(x), got)
             layer._fused_forward = fused
+
+
+def test_graphs_outlive_other_streams(cuda_device):
+    """A graph per stream, each after a warm-up on that stream, then passes on yet other streams: replays of every graph still
+    read the tensor scales that they were captured with, although the memory of whatever was dropped has been reused."""
+    layer = _layer(cuda_device, 384, 256, "NVFP4", "abs_max", 16, torch.bfloat16)
+    x = torch.randn(40, 384, device=cuda_device).bfloat16()
+    graphs, streams = [], []
+    with torch.no_grad():
+        want = layer(x).clone()
+        for _ in range(10):
+            stream = torch.cuda.Stream()
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                layer(x)
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                y = layer(x)
+            graphs.append((graph, y))
+            streams.append(stream)
+            with torch.cuda.stream(stream):             # takes up whatever small blocks this stream's sets left
+                streams.append([torch.full((1,), 1e4, device=cuda_device) for _ in range(40)])
+        streams.append([torch.full((1,), 1e4, device=cuda_device) for _ in range(200)])
+        for graph, y in graphs:
+            y.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("fmt,backward", [("MXFP4", "MXFP8"), ("MXFP4", "MXFP4"), ("NVFP4", "BF16")])
+def test_replayed_training_steps_follow_the_tensor_scales(cuda_device, fmt, backward):
+    """A graph of a training step derives what it needs from the two tensor scales itself: a replay after an update in place
+    gives what an eager step gives."""
+    k, n = 384, 256
+    layer = _layer(cuda_device, k, n, fmt, "abs_max", 16 if fmt == "NVFP4" else 32, None, backward=backward, master=True)
+    x = torch.randn(128, k, device=cuda_device).bfloat16().requires_grad_(True)
+    g = torch.randn(128, n, device=cuda_device).bfloat16() * 0.01
+
+    def step():
+        return torch.autograd.grad((y := layer(x)), (x, layer.weight), g) + (y.detach(),)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            step()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step()
+    with torch.no_grad():
+        layer.weight_global_scale.mul_(0.5)
+        layer.act_global_scale.mul_(0.25)
+    want = step()
+    graph.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(out, want):
+        assert torch.equal(a, b)
