@@ -13,19 +13,13 @@ from torch.autograd import Function
 
 from ..utils.config import FPQuantDtype
 from ... import ops
+from ...ops import plain_eager
 from ...rotation import kind_of
 from .qutlass_ops import (backward_bf16_square_double_mxfp8_op, backward_qt_bf16_op, backward_t_bf16_op,
                           fused_quantize_blocked_op, fused_quantize_mx_op,
                           fused_quantize_nv_op, matmul_fp4_bf16_tn_blocked_op, matmul_mxf4_bf16_tn_op,
                           matmul_mxf8_bf16_nn_op, matmul_mxf8_bf16_tn_op, matmul_nvf4_bf16_tn_op,
                           mxfp4_transpose_mxfp8_op)
-
-
-def plain_eager(x: torch.Tensor) -> bool:
-    """No tracer, dispatch mode, functorch transform or tensor subclass between the caller and the kernels: the native calls
-    may be made without the registered ops (85 us of dispatch each)."""
-    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._functorch.peek_interpreter_stack() is None)
 
 
 class GemmConstants:

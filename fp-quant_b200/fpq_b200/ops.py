@@ -5,12 +5,27 @@ from __future__ import annotations
 from typing import Optional, Tuple
 
 import torch
+from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
+from torch._C._functorch import peek_interpreter_stack
+from torch.autograd import forward_ad
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _cabi as C
 from ._cabi import call as _cabi_call
 
 FORMATS = {"mxfp4": C.FMT_MXFP4, "nvfp4": C.FMT_NVFP4}
 GROUP_OF = {"mxfp4": 32, "nvfp4": 16}
+
+
+def plain_eager(x: torch.Tensor) -> bool:
+    """No tracer, dispatch or function mode (but the one that sets a default device), functorch transform, forward-mode
+    derivative or tensor subclass between the caller and the kernels: native calls may be made on x's address without
+    the registered ops (85 us of dispatch each)."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
+            and _len_torch_dispatch_stack() == 0 and peek_interpreter_stack() is None and forward_ad._current_level < 0
+            and (_len_torch_function_stack() == 0
+                 or all(type(m) is DeviceContext for m in _get_current_function_mode_stack())))
 
 
 def _dt(t: torch.Tensor) -> int:

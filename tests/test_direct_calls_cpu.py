@@ -1,10 +1,52 @@
-"""What a layer keeps between passes."""
+"""When the native calls may be made on a tensor's address, and what a layer keeps between passes."""
 import threading
 import weakref
 
+import pytest
 import torch
+import torch.autograd.forward_ad as forward_ad
+from torch.overrides import TorchFunctionMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from fpq_b200.fp_quant.module.linear_fns import ConstantsCache
+from fpq_b200.ops import plain_eager
+
+
+class _Functions(TorchFunctionMode):
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+class _Dispatch(TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        return func(*args, **(kwargs or {}))
+
+
+class _Subclass(torch.Tensor):
+    pass
+
+
+def test_plain_eager():
+    x = torch.ones(2, 32)
+    assert plain_eager(x) and plain_eager(torch.nn.Parameter(x))
+    with torch.device("cpu"):                     # sets a default for factories, sees nothing else
+        assert plain_eager(x)
+    for mode in (_Functions(), _Dispatch(), forward_ad.dual_level()):
+        with mode:
+            assert not plain_eager(x)
+    with torch.device("cpu"), _Functions():
+        assert not plain_eager(x)
+    assert not plain_eager(x.as_subclass(_Subclass))
+    seen = []
+
+    def look(t):
+        seen.append(plain_eager(t))
+        return t
+
+    torch.func.vmap(look)(x)
+    torch.func.jvp(look, (x,), (x,))
+    torch.compile(look, backend="eager", fullgraph=True)(x)
+    assert not any(seen) and len(seen) == 3
 
 
 def _scales():
