@@ -5,11 +5,7 @@ from __future__ import annotations
 from typing import Optional, Tuple
 
 import torch
-from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
-from torch._C._functorch import peek_interpreter_stack
 from torch.autograd import forward_ad
-from torch.overrides import _get_current_function_mode_stack
-from torch.utils._device import DeviceContext
 
 from . import _cabi as C
 from ._cabi import call as _cabi_call
@@ -18,11 +14,22 @@ FORMATS = {"mxfp4": C.FMT_MXFP4, "nvfp4": C.FMT_NVFP4}
 GROUP_OF = {"mxfp4": 32, "nvfp4": 16}
 
 
+try:        # private names of torch: where one is missing, the calls below take the general way
+    from torch._C import _len_torch_dispatch_stack, _len_torch_function_stack
+    from torch._C._functorch import peek_interpreter_stack
+    from torch.overrides import _get_current_function_mode_stack
+    from torch.utils._device import DeviceContext
+    forward_ad._current_level
+    _CAN_TELL = True
+except (ImportError, AttributeError):
+    _CAN_TELL = False
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def plain_eager(x: torch.Tensor) -> bool:
     """No tracer, dispatch or function mode (but the one that sets a default device), functorch transform, forward-mode
-    derivative or tensor subclass between the caller and the kernels: native calls may be made on x's address without
-    the registered ops (85 us of dispatch each)."""
-    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
+    derivative or tensor subclass between the caller and the kernels: native calls may be made on x's address."""
+    return (_CAN_TELL and type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
             and _len_torch_dispatch_stack() == 0 and peek_interpreter_stack() is None and forward_ad._current_level < 0
             and (_len_torch_function_stack() == 0
                  or all(type(m) is DeviceContext for m in _get_current_function_mode_stack())))
@@ -43,7 +50,9 @@ def _cuda(t: torch.Tensor, name: str = "tensor") -> torch.Tensor:
 
 
 def _stream(t: torch.Tensor) -> int:
-    return torch._C._cuda_getCurrentRawStream(t.device.index)     # without building a Stream object (1 us of 1.2)
+    if _raw_stream is None:
+        return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.device.index)     # without building a Stream object (1 us of 1.2)
 
 
 class _NoGuard:

@@ -1,8 +1,10 @@
 """When the native calls may be made on a tensor's address, and what a layer keeps between passes."""
+import os
+import subprocess
+import sys
 import threading
 import weakref
 
-import pytest
 import torch
 import torch.autograd.forward_ad as forward_ad
 from torch.overrides import TorchFunctionMode
@@ -47,6 +49,22 @@ def test_plain_eager():
     torch.func.jvp(look, (x,), (x,))
     torch.compile(look, backend="eager", fullgraph=True)(x)
     assert not any(seen) and len(seen) == 3
+
+
+def test_another_torch_without_the_private_names():
+    """The package loads, takes the general way and asks for the stream through the public call."""
+    code = """
+import sys, torch, types
+for name in ("_len_torch_function_stack", "_cuda_getCurrentRawStream"):
+    if hasattr(torch._C, name):
+        delattr(torch._C, name)
+from fpq_b200 import ops
+assert not ops.plain_eager(torch.ones(2))
+torch.cuda.current_stream = lambda device: types.SimpleNamespace(cuda_stream=(device, 7))
+t = types.SimpleNamespace(device=torch.device("cuda", 1))
+assert ops._stream(t) == (t.device, 7)
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, env={**os.environ, "PYTHONPATH": os.pathsep.join(sys.path)})
 
 
 def _scales():
