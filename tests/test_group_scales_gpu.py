@@ -73,3 +73,37 @@ def test_checks_of_the_scales(cuda_device, fmt):
         q.get_quantization_params(torch.zeros_like(x))
         with pytest.raises(ValueError):
             q.raise_deferred_checks()
+
+
+def test_dequantize_under_modes_and_transforms(cuda_device):
+    """The product of `dequantize` where its kernel must not be called on an address: vmap, a dispatch mode that records it,
+    make_fx, torch.compile without graph breaks and forward-mode derivatives."""
+    import torch.autograd.forward_ad as forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from fpq_b200.quantization.quantizer import Quantizer
+
+    quantizer = Quantizer(bits=4, symmetric=True, format="mxfp", granularity="group", group_size=32, scale_precision="e8m0")
+    q = torch.randint(-6, 7, (6, 96), device=cuda_device).float()
+    s = torch.rand(6, 3, device=cuda_device) + 0.1
+    want = q * s.repeat_interleave(32, dim=1)
+    assert torch.equal(quantizer.dequantize(q, s), want)
+    assert torch.equal(torch.func.vmap(quantizer.dequantize)(q.view(2, 3, 96), s.view(2, 3, 3)).view(6, 96), want)
+    seen = []
+
+    class Record(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    with Record():
+        assert torch.equal(quantizer.dequantize(q, s), want)
+    assert any("mul" in f for f in seen)
+    traced = make_fx(lambda a, b: quantizer.dequantize(a, b))(q, s)
+    assert torch.equal(traced(2 * q, s), 2 * want)
+    assert torch.equal(torch.compile(quantizer.dequantize, backend="eager", fullgraph=True)(q, s), want)
+    with forward_ad.dual_level():
+        dual = quantizer.dequantize(forward_ad.make_dual(q, torch.ones_like(q)), s)
+        tangent = forward_ad.unpack_dual(dual).tangent
+        assert torch.equal(tangent, s.repeat_interleave(32, dim=1))
