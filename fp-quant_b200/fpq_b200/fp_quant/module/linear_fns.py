@@ -257,17 +257,20 @@ def _mxfp8_backward(grad_output, x_q, w_q, x_scales, w_scales, act_global_scale,
 
 
 def _training_forward(x, weight, weight_global_scale, act_global_scale, bias, hadamard_matrix, dtype, forward_method,
-                      constants: Optional[GemmConstants], direct: bool = True):
+                      constants: Optional[GemmConstants], mxfp4_backward: bool = False):
     """Forward pass of the MXFP4 layers whose backward runs on quantised operands: (y, (codes, scales, clip mask) of x and
-    of the weight, whether the scales are swizzled).  Where `direct` allows it and the calls need not be traced, the
-    kernels are called directly and the scales stay in the layout that the matmul reads; otherwise the reference's op
-    sequence with its row-major scales."""
+    of the weight, whether the scales are swizzled).  Where the calls need not be traced and the backward (the MXFP4 one has
+    a general form) reads the scales so, the kernels are called directly and the scales stay in the layout that the
+    matmul reads; otherwise the reference's op sequence with its row-major scales.  The rotation is classified once: that
+    waits for the GPU where the matrix has to be converted (weights that are not bf16)."""
     x_flat = x.contiguous().flatten(end_dim=-2)
     matrix = hadamard_matrix.to(torch.bfloat16)
-    direct = (direct and constants is not None and dtype == FPQuantDtype.MXFP4 and forward_method in ("abs_max", "quest")
-              and plain_eager(x) and plain_eager(weight) and kind_of(0, matrix)[0] != "dense")
+    direct = (constants is not None and dtype == FPQuantDtype.MXFP4 and forward_method in ("abs_max", "quest")
+              and plain_eager(x) and plain_eager(weight))
     if direct:
         kind, group = kind_of(0, matrix)
+        direct = kind != "dense" and (not mxfp4_backward or _fused_mxfp4_backward(kind, group, weight.shape[0]))
+    if direct:
         group = group if kind == "hadamard" else 0
 
         def quantize(t):
@@ -279,8 +282,8 @@ def _training_forward(x, weight, weight_global_scale, act_global_scale, bias, ha
         xq, wq = quantize(x_flat), quantize(weight)
         y = ops.gemm_fp4(xq[0], wq[0], xq[1], wq[1], constants.alpha, "mxfp4")
     else:
-        xq = forward_quantize(x_flat, hadamard_matrix, act_global_scale, dtype, forward_method)
-        wq = forward_quantize(weight, hadamard_matrix, weight_global_scale, dtype, forward_method)
+        xq = forward_quantize(x_flat, matrix, act_global_scale, dtype, forward_method)
+        wq = forward_quantize(weight, matrix, weight_global_scale, dtype, forward_method)
         y = forward_gemm(xq[0], wq[0], xq[1], wq[1], 1.0 / (weight_global_scale * act_global_scale), dtype)
     y = y.unflatten(dim=0, sizes=x.shape[:-1])
     if bias is not None:
@@ -288,9 +291,8 @@ def _training_forward(x, weight, weight_global_scale, act_global_scale, bias, ha
     return y, xq, wq, direct
 
 
-def _fused_mxfp4_backward(hadamard_matrix: torch.Tensor, out_features: int) -> bool:
+def _fused_mxfp4_backward(kind: str, group: int, out_features: int) -> bool:
     """Whether the MXFP4 backward runs on the transposing kernels: a rotation that fits a scale group, rows they can load."""
-    kind, group = kind_of(0, hadamard_matrix.to(torch.bfloat16))
     return kind in ("hadamard", "identity") and group <= 32 and out_features % 8 == 0
 
 
@@ -348,7 +350,7 @@ class FPQuant4x4MasterFn(Function):
                 forward_method, constants: Optional[GemmConstants] = None):
         y, (x_q, x_scales, x_mask), (w_q, w_scales, w_mask), ctx.swizzled = _training_forward(
             x, weight, weight_global_scale, act_global_scale, bias, forward_hadamard_matrix, dtype, forward_method, constants,
-            direct=_fused_mxfp4_backward(forward_hadamard_matrix, weight.shape[0]))
+            mxfp4_backward=True)
         ctx.x_shape, ctx.bias_present, ctx.constants = x.shape, bias is not None, constants
         ctx.masks = (x_mask, w_mask)
         ctx.save_for_backward(x_q, w_q, x_scales, w_scales, act_global_scale, weight_global_scale, forward_hadamard_matrix)
@@ -370,7 +372,7 @@ class FPQuant4x4MasterFn(Function):
         # abs_max MXFP4 carries a factor 3 per operand (the scale is a third of the power of two that is stored)
         ninth = torch.full((1,), 1.0 / 9.0, dtype=torch.float32, device=g.device)
         kind, group = kind_of(0, backward_hadamard_matrix)
-        if _fused_mxfp4_backward(hadamard_matrix, out_features):
+        if _fused_mxfp4_backward(kind, group, out_features):
             # Same data flow as the op sequence below with the re-layouts folded into the producers: scales come
             # out in the layout the GEMM reads, the transposes happen inside the (de)quantise kernels, and the
             # token axis is padded to a whole number of K tiles by the kernels that write it.

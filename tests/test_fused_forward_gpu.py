@@ -84,6 +84,25 @@ def test_training_matches_the_general_path(cuda_device, fmt, backward, method, g
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("backward", ["MXFP8", "MXFP4"])
+@pytest.mark.parametrize("group", [32, 64])
+def test_rotation_of_fp32_layers_is_classified_once_a_pass(cuda_device, monkeypatch, backward, group):
+    """A matrix that has to be converted to bf16 is a new tensor on every pass, and classifying it waits for the GPU: at most one
+    wait in the forward and one in the backward, whatever path the rotation takes."""
+    from fpq_b200 import rotation
+
+    layer = _layer(cuda_device, 384, 256, "MXFP4", "quest", group, backward=backward, master=True, dtype=torch.float32)
+    x = torch.randn(64, 384, device=cuda_device, requires_grad=True)
+    layer(x).sum().backward()
+    waits = []
+    sylvester = rotation.sylvester
+    monkeypatch.setattr(rotation, "sylvester", lambda g: (waits.append(g), sylvester(g))[1])
+    y = layer(x)
+    assert len(waits) <= 1
+    y.sum().backward()
+    assert len(waits) <= 2
+
+
 def test_long_products_and_other_streams(cuda_device):
     """Above the size where quantise and GEMM become two calls; passes on a stream of their own and from a graph that was
     captured before any eager pass."""
