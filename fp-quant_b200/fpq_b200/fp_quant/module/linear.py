@@ -65,6 +65,11 @@ class FPQuantLinear(nn.Module):
         self._scales_blocked_key = None
         self._constants = ConstantsCache()
 
+    def __setstate__(self, state):
+        """A copy or an unpickled layer makes its constants anew (layers saved by earlier versions have none)."""
+        super().__setstate__(state)
+        self.__dict__["_constants"] = ConstantsCache()
+
     # ------------------------------------------------------------------ load-time step
     @torch.no_grad()
     def pre_forward(self):

@@ -1,5 +1,7 @@
 """When the native calls may be made on a tensor's address, and what a layer keeps between passes."""
+import copy
 import os
+import pickle
 import subprocess
 import sys
 import threading
@@ -127,3 +129,20 @@ def test_constants_follow_the_scales():
     for t in threads:
         t.join()
     assert not errors
+
+
+def test_layers_saved_without_constants_load():
+    """A layer pickled whole before it kept constants, and a copy of a layer that has handed some to a capture."""
+    from fpq_b200.fp_quant import FPQuantConfig, FPQuantDtype, FPQuantLinear
+
+    layer = FPQuantLinear(64, 32, FPQuantConfig(forward_dtype=FPQuantDtype.MXFP4), device="cpu", dtype=torch.bfloat16)
+    with torch.no_grad():
+        layer.weight_global_scale.fill_(3)
+        layer.act_global_scale.fill_(3)
+    want = float(layer._gemm_alpha())
+    layer._constants.get(layer.weight_global_scale, layer.act_global_scale, 0, True)
+    twin = copy.deepcopy(layer)
+    assert float(twin._gemm_alpha()) == want and not twin._constants._captured
+    del layer._constants
+    loaded = pickle.loads(pickle.dumps(layer))
+    assert float(loaded._gemm_alpha()) == want
