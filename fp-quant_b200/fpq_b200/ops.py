@@ -365,6 +365,12 @@ def gemm_fp4(a_codes: torch.Tensor, b_codes: torch.Tensor, a_scales_swizzled: to
     return out
 
 
+def linear_workspace_bytes(m: int, k: int, nvfp4: bool) -> int:
+    """fpq_linear_workspace_bytes, without a native call on every pass."""
+    sf_cols = k // 16 if nvfp4 else k // 32
+    return ((m * (k // 2) + 255) & -256) + ((m + 127) & -128) * ((sf_cols + 3) & -4)
+
+
 def linear_forward(x: torch.Tensor, up: Optional[torch.Tensor], w_codes: torch.Tensor, w_scales_swizzled: torch.Tensor,
                    alpha: torch.Tensor, fmt: str, hadamard_group: int, quest: bool, global_scale: Optional[torch.Tensor],
                    bias: Optional[torch.Tensor]) -> torch.Tensor:
@@ -386,8 +392,7 @@ def linear_forward(x: torch.Tensor, up: Optional[torch.Tensor], w_codes: torch.T
         else:
             q, sb, _ = quantize(x2, fmt, hadamard_group, global_scale if nv else None, swizzled=True)
         return gemm_fp4(q, w_codes, sb, w_scales_swizzled, alpha, fmt, bias).view(x.shape[:-1] + (n,))
-    sf_cols = k // 16 if nv else k // 32
-    size = ((m * k // 2 + 255) & -256) + ((m + 127) & -128) * ((sf_cols + 3) & -4)
+    size = linear_workspace_bytes(m, k, nv)
     dev = x.device
     ws = torch.empty(size, dtype=torch.uint8, device=dev)
     out = torch.empty(x.shape[:-1] + (n,), dtype=torch.bfloat16, device=dev)

@@ -38,6 +38,18 @@ def test_every_declaration_cites_the_reference():
         assert re.search(r"\.py:\d+", comment) or "no counterpart in the reference" in comment, name
 
 
+@pytest.mark.parametrize("nvfp4", [False, True])
+def test_linear_workspace_is_the_librarys(nvfp4):
+    """The size that the one-call forward allocates, over odd row counts and scale columns off the multiple of four."""
+    from fpq_b200 import _cabi as C
+    from fpq_b200 import ops
+
+    for m in (1, 2, 63, 127, 128, 129, 3001, 16384):
+        for k in (32, 64, 96, 160, 1024, 4128, 17408):
+            want = C.lib().fpq_linear_workspace_bytes(m, k, C.FMT_NVFP4 if nvfp4 else C.FMT_MXFP4)
+            assert ops.linear_workspace_bytes(m, k, nvfp4) == want
+
+
 def test_no_cpu_fallback():
     from fpq_b200 import ops
 
