@@ -489,11 +489,6 @@ __global__ void __launch_bounds__(256) transpose_split3_kernel(const float* __re
 
 int64_t round64(int64_t x) { return (x + 63) & ~(int64_t)63; }
 
-// bf16 elements of workspace tc_gemm3 needs
-int64_t tc_gemm3_workspace(int64_t M, int64_t N, int64_t K, bool b_is_a_transposed) {
-  return 3 * K * round64(M) + (b_is_a_transposed ? 0 : 3 * K * round64(N));
-}
-
 // C[M, N] (row stride ldc) = beta * C + alpha * A B with fp32-level accuracy on the tensor cores:
 // A [M, K] row-major (lda); B [K, N] row-major (ldb), or B == nullptr for B = (the first N rows of A)^T:
 // with N == M the symmetric rank-K update (only the tiles touching the lower triangle are computed), with

@@ -749,11 +749,11 @@ __device__ __forceinline__ uint32_t silu_mul_word(uint32_t g2, uint32_t u2) {
 // The same for the sixteen words of a chunk whose gates all lie in [-80, 80], two elements per instruction:
 //   t = 2^(-g log2 e): log2 e = C1 + C2 with C1 of 16 bits, so that g C1 is exact (g has 8 bits); what is
 //   left is 2^(-g C2) = 1 - g C2 ln 2 (within 2^-23 at |g| = 80, less below) and the error of ex2.approx;
-//   g / (1 + t) by reciprocal and one fused residual correction.
+//   g / (1 + t) by reciprocal and one fused residual correction (Markstein, IBM J. Res. Dev. 34, 1990).
 // t is raised by 2^-25: silu(2^-7) lies 5e-6 of a bf16 unit below a rounding tie, where fp32 has to land on the tie as
 // the library's does (every raise from 2^-26 to 2^-23 agrees on all inputs, none at all misses this one).
 // silu is a function of 16 input bits here: the rounded result equals the library exponential with the IEEE division on
-// every one of them, which a test checks.  5.5 instructions an element instead of about 25: the kernel, bound by
+// every one of them, which a test checks for all gates up to 80.  5.5 instructions an element instead of about 25: the kernel, bound by
 // instruction issue before, takes 137 us instead of 215 for 8192 x 17408 (MXFP4, rotation 32; 4.7 TB/s of 6.5).
 __device__ __forceinline__ void silu_mul_chunk(const RawChunk<true>& g, const RawChunk<true>& u, RawChunk<true>& h) {
   const u64 NC1 = pack2(-1.44268798828125f, -1.44268798828125f);            // -(log2 e rounded to 16 bits)

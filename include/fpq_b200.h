@@ -92,7 +92,8 @@ int fpq_absmax(const void* x, int dtype, int64_t rows, int64_t cols, int hadamar
 /*
  * *global_scale = min(*global_scale, fl(2688 * fl(1 / absmax))) -- the running-min
  * update of Quantizer.global_scale (src/quantization/quantizer.py:10-16, :145-150).
- * A zero absmax leaves the scale unchanged and sets *status to 1.
+ * A zero absmax leaves the scale unchanged.  *status (optional) becomes 1 then and when the new scale is not finite,
+ * else 0.
  */
 int fpq_global_scale_update(const uint32_t* absmax_bits, float* global_scale, int32_t* status,
                             fpq_stream_t stream);

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from fpq_b200.fp_quant import FPQuantConfig, FPQuantDtype, FPQuantLinear
+from fpq_b200.fp_quant.module import linear_fns
 
 pytestmark = pytest.mark.gpu
 
@@ -36,6 +37,7 @@ def test_inference_matches_the_general_path(cuda_device, fmt, method, group, tra
             for x in forms:
                 got = layer(x)
                 fused = layer._fused_forward
+                assert (fused(x) is not None) == (transform != "gsr" and bias is not torch.float32)
                 layer._fused_forward = lambda *a: None
                 want = layer(x)
                 layer._fused_forward = fused
@@ -44,6 +46,7 @@ def test_inference_matches_the_general_path(cuda_device, fmt, method, group, tra
                 for m in (1, 65, 300):
                     g, u = base[:m], torch.randn(m, k, device=cuda_device).bfloat16()
                     got = layer.forward_silu_mul(g, u)
+                    assert (fused(g, u) is not None) == (bias is not torch.float32)
                     layer._fused_forward = lambda *a: None
                     want = layer.forward_silu_mul(g, u)
                     layer._fused_forward = fused
@@ -65,13 +68,21 @@ def test_inference_matches_the_general_path(cuda_device, fmt, method, group, tra
                                                        ("MXFP4", "MXFP4", "quest", 32), ("MXFP4", "MXFP4", "abs_max", 64),
                                                        ("NVFP4", "BF16", "abs_max", 16), ("MXFP4", "BF16", "quest", 32)])
 @pytest.mark.parametrize("tokens", [(64,), (2, 77)])
-def test_training_matches_the_general_path(cuda_device, fmt, backward, method, group, tokens):
+def test_training_matches_the_general_path(cuda_device, monkeypatch, fmt, backward, method, group, tokens):
     """Same kernels on the same operands: output and gradients bit for bit."""
     k, n = 384, 256
     layer = _layer(cuda_device, k, n, fmt, method, group, torch.bfloat16, backward=backward, master=True)
     x = torch.randn(*tokens, k, device=cuda_device).bfloat16()
     g = torch.randn(*tokens, n, device=cuda_device).bfloat16() * 0.01
-    out = []
+    out, direct = [], []
+    training_forward = linear_fns._training_forward
+
+    def watch(*args, **kwargs):
+        result = training_forward(*args, **kwargs)
+        direct.append(result[3])
+        return result
+
+    monkeypatch.setattr(linear_fns, "_training_forward", watch)
     for general in (False, True):
         if general:
             layer._training_constants = lambda x: None
@@ -82,6 +93,8 @@ def test_training_matches_the_general_path(cuda_device, fmt, backward, method, g
         out.append((y, xi.grad, layer.weight.grad, layer.bias.grad))
     for a, b in zip(*out):
         assert torch.equal(a, b)
+    # the kernels directly, then the registered ops; the MXFP4 backward reads swizzled scales up to a rotation of 32 alone
+    assert direct == ([] if backward == "BF16" else [not (backward == "MXFP4" and group > 32), False])
 
 
 @pytest.mark.parametrize("backward", ["MXFP8", "MXFP4"])

@@ -73,6 +73,16 @@ def test_checks_of_the_scales(cuda_device, fmt):
         q.get_quantization_params(torch.zeros_like(x))
         with pytest.raises(ValueError):
             q.raise_deferred_checks()
+        # a NaN among the group scales, at once and deferred: no longer tracked, the tensor scale is not looked at itself
+        for deferred in (False, True):
+            q = make()
+            q.get_quantization_params(x)
+            q._track_global_scale = False
+            q.global_scale.fill_(float("nan"))
+            q.deferred_checks = [] if deferred else None
+            with pytest.raises(ValueError, match="Scales"):
+                q.get_quantization_params(x)
+                q.raise_deferred_checks()
 
 
 def test_dequantize_under_modes_and_transforms(cuda_device):
