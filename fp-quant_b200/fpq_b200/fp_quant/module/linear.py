@@ -129,12 +129,12 @@ class FPQuantLinear(nn.Module):
             self._scales_blocked_key = key
         return self._scales_blocked
 
-    def _gemm_constants(self, training: bool = False) -> GemmConstants:
-        """What the passes derive from the two tensor scales (see `ConstantsCache`)."""
+    def _gemm_constants(self) -> GemmConstants:
+        """What an inference pass derives from the two tensor scales (see `ConstantsCache`)."""
         w, a = self.weight_global_scale, self.act_global_scale
         if not w.is_cuda:
-            return self._constants.get(w, a, 0, False)
-        return self._constants.get(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing(), follow=training)
+            return self._constants.inference(w, a, 0, lambda: False)
+        return self._constants.inference(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing)
 
     def _gemm_alpha(self) -> torch.Tensor:
         """1 / (weight_global_scale * act_global_scale) as fp32 [1]."""
@@ -199,8 +199,13 @@ class FPQuantLinear(nn.Module):
         return y.unflatten(dim=0, sizes=lead)
 
     def _training_constants(self, x: torch.Tensor):
-        """The cached constants for a training pass; None (they are derived on the way) under a tracer."""
-        return self._gemm_constants(training=True) if plain_eager(x) else None
+        """The constants for a training pass; None (they are derived on the way) under a tracer."""
+        if not plain_eager(x):
+            return None
+        w, a = self.weight_global_scale, self.act_global_scale
+        if not w.is_cuda:
+            return self._constants.training(w, a, 0, False)
+        return self._constants.training(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing())
 
     # ------------------------------------------------------------------ forward
     def forward(self, x) -> torch.Tensor:

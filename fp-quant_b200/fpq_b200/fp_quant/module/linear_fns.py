@@ -6,7 +6,7 @@ weights raises like the reference does.  `FPQuant4x4MasterFn` runs both gradient
 """
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import Callable, Optional, Tuple
 
 import torch
 from torch.autograd import Function
@@ -27,9 +27,19 @@ class GemmConstants:
     MXFP8 backward their inverses, made when they are first asked for."""
 
     @torch.no_grad()
-    def __init__(self, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor):
+    def __init__(self, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor, own: bool = False):
+        """`own`: never the storage of fp32 scales themselves, so that `update` can be called."""
         self.alpha = gemm_alpha(weight_global_scale, act_global_scale)
-        self.weight_scale, self.act_scale = weight_global_scale.float().reshape(1), act_global_scale.float().reshape(1)
+        self.weight_scale, self.act_scale = (s.to(torch.float32, copy=own).reshape(1)
+                                             for s in (weight_global_scale, act_global_scale))
+        self._inverses = None
+
+    @torch.no_grad()
+    def update(self, weight_global_scale: torch.Tensor, act_global_scale: torch.Tensor) -> None:
+        """The same tensors with the values of other scales."""
+        self.alpha.copy_(gemm_alpha(weight_global_scale, act_global_scale))
+        self.weight_scale.copy_(weight_global_scale.reshape(1))
+        self.act_scale.copy_(act_global_scale.reshape(1))
         self._inverses = None
 
     @torch.no_grad()
@@ -47,36 +57,58 @@ class GemmConstants:
 class ConstantsCache:
     """`GemmConstants` of one layer, remade only when one of its two tensor scales changed (up to nine small kernels per
     training step otherwise).  The tensors a set was made from are kept and compared as objects, so an address that is used
-    again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written yet."""
+    again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written yet.
+    Nothing made while the stream is being captured is kept: its values only exist after a replay."""
+    STREAMS = 8
 
     def __init__(self):
-        self._of = None         # (key, {stream: set}), replaced as a whole: threads see one state or the other
-        self._captured = []     # sets whose addresses a CUDA graph holds: kept for as long as the layer lives
+        self._training = None       # (scales, {stream: set}), replaced as a whole: threads see one state or the other
+        self._inference = {}        # stream: [scales, set], the sets for as long as the layer lives
 
-    def get(self, w: torch.Tensor, a: torch.Tensor, stream: int, capturing: bool, follow: bool = False) -> GemmConstants:
-        """The set for a pass on `stream`.  While that stream is being captured: with `follow` a set of the graph's own, whose
-        replays follow the scales (training passes, whose scales may be updated in place); else the set of an earlier
-        pass, which costs the replays nothing, frozen as it is now.  Nothing made inside a capture is kept: its values
-        only exist after a replay."""
-        if capturing and follow:
+    @staticmethod
+    def _same(of, w: torch.Tensor, a: torch.Tensor) -> bool:
+        return (of[0] is w and of[1] is a and of[2] == w._version and of[3] == a._version and of[4] == w.data_ptr()
+                and of[5] == a.data_ptr())
+
+    @staticmethod
+    def _of(w: torch.Tensor, a: torch.Tensor):
+        return (w, a, w._version, a._version, w.data_ptr(), a.data_ptr())
+
+    def training(self, w: torch.Tensor, a: torch.Tensor, stream: int, capturing: bool) -> GemmConstants:
+        """A set that stays as it is, since a backward pass may hold it.  A captured step derives its own inside the graph:
+        replays follow updates of the scales in place, and no graph holds an address in here."""
+        if capturing:
             return GemmConstants(w, a)
-        of = self._of
-        key = (w._version, a._version, w.data_ptr(), a.data_ptr())
-        if of is None or of[0] is not w or of[1] is not a or of[2] != key:
-            of = self._of = (w, a, key, {})
-        kept = of[3]
+        state = self._training
+        if state is None or not self._same(state[0], w, a):
+            state = self._training = (self._of(w, a), {})
+        kept = state[1]
         consts = kept.get(stream)
-        if not capturing:
-            if consts is None:
-                if len(kept) >= 8:
-                    kept.clear()
-                consts = kept[stream] = GemmConstants(w, a)
-            return consts
-        consts = consts or next(iter(kept.values()), None)
         if consts is None:
+            if len(kept) >= self.STREAMS:
+                kept.clear()
+            consts = kept[stream] = GemmConstants(w, a)
+        return consts
+
+    def inference(self, w: torch.Tensor, a: torch.Tensor, stream: int, capturing: Callable[[], bool]) -> GemmConstants:
+        """A set that CUDA graphs may hold the addresses of: captured passes take an earlier pass's, which costs their replays
+        nothing.  It is therefore never dropped, and new scales are written into it.  `capturing` is only asked where this
+        stream's set does not fit (the question costs a decode step a microsecond)."""
+        entry = self._inference.get(stream)
+        if entry is not None and self._same(entry[0], w, a):
+            return entry[1]
+        if capturing():
+            for of, consts in list(self._inference.values()):
+                if self._same(of, w, a):
+                    return consts
             return GemmConstants(w, a)
-        if not any(c is consts for c in self._captured):
-            self._captured.append(consts)
+        if entry is not None and entry[1].alpha.device == w.device:
+            entry[1].update(w, a)
+            entry[0] = self._of(w, a)
+            return entry[1]
+        consts = GemmConstants(w, a, own=True)
+        if entry is not None or len(self._inference) < self.STREAMS:
+            self._inference[stream] = [self._of(w, a), consts]
         return consts
 
 

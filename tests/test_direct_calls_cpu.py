@@ -73,51 +73,74 @@ def _scales():
     return torch.tensor([3.0], dtype=torch.bfloat16), torch.tensor([3.0], dtype=torch.bfloat16)
 
 
+def _yes():
+    return True
+
+
+def _no():
+    return False
+
+
 def test_a_captured_graphs_constants_outlive_other_streams_and_new_scales():
-    """What a capture was given stays alive with the cache, whatever streams and scales come after."""
+    """What a captured inference pass was given stays alive with the cache and at its address, whatever streams and scales
+    come after, and holds the values of new scales once a pass has seen them on the set's stream."""
     w, a = _scales()
     cache = ConstantsCache()
-    own = cache.get(w, a, 1, False)
-    held = [weakref.ref(cache.get(w, a, 1, True)), weakref.ref(cache.get(w, a, 2, True))]     # its own stream's set, another's
-    assert held[0]() is own and held[1]() is own
-    kept = weakref.ref(cache.get(w, a, 3, False))
+    own = cache.inference(w, a, 1, _no)
+    assert cache.inference(w, a, 1, _yes) is own and cache.inference(w, a, 2, _yes) is own     # its own stream's, another's
+    held, address = weakref.ref(own), [t.data_ptr() for t in (own.alpha, own.act_scale, own.weight_scale)]
     del own
-    for stream in range(4, 24):
-        assert cache.get(w, a, stream, False) is cache.get(w, a, stream, False)
+    for stream in range(2, 24):
+        assert float(cache.inference(w, a, stream, _no).alpha) == float((1.0 / (w * a)).float())
+    assert len(cache._inference) == cache.STREAMS
     w.mul_(2)
-    for stream in range(1, 24):
-        assert float(cache.get(w, a, stream, False).alpha) == float((1.0 / (w * a)).float())
-    assert all(r() is not None for r in held) and kept() is None
-    assert len(cache._of[3]) <= 8
+    fresh = cache.inference(w, a, 1, _yes)                 # no set of the new scales yet: the graph's own
+    assert fresh is not held() and float(held().weight_scale) == 3.0
+    other = torch.tensor([5.0], dtype=torch.bfloat16)
+    for scale in (w, other):
+        for stream in range(1, 24):
+            got = cache.inference(scale, a, stream, _no)
+            assert float(got.weight_scale) == float(scale) and float(got.alpha) == float((1.0 / (scale * a)).float())
+        assert cache.inference(scale, a, 1, _no) is held() and float(held().weight_scale) == float(scale)
+    assert [t.data_ptr() for t in (held().alpha, held().act_scale, held().weight_scale)] == address
+
+
+def test_sets_do_not_write_into_fp32_scales():
+    w, a = torch.tensor([3.0]), torch.tensor([2.0])
+    cache = ConstantsCache()
+    cache.inference(w, a, 1, _no)
+    other = torch.tensor([7.0])
+    assert float(cache.inference(other, a, 1, _no).weight_scale) == 7.0
+    assert float(w) == 3.0
 
 
 def test_what_a_capture_makes_is_not_kept():
     w, a = _scales()
     cache = ConstantsCache()
-    first = cache.get(w, a, 1, True)                       # no earlier pass: made inside the graph
-    assert cache.get(w, a, 1, False) is not first
-    eager = cache.get(w, a, 1, False)
-    follow = cache.get(w, a, 1, True, follow=True)         # a training step's graph derives its own
-    assert follow is not eager and cache.get(w, a, 1, False) is eager
+    first = cache.inference(w, a, 1, _yes)                 # no earlier pass: made inside the graph
+    assert cache.inference(w, a, 1, _no) is not first
+    eager = cache.training(w, a, 1, False)
+    follow = cache.training(w, a, 1, True)                 # a training step's graph derives its own
+    assert follow is not eager and cache.training(w, a, 1, False) is eager
 
 
-def test_constants_follow_the_scales():
+def test_training_constants_follow_the_scales_and_stay_as_they_are():
     w, a = _scales()
     cache = ConstantsCache()
-    first = cache.get(w, a, 1, False)
-    assert cache.get(w, a, 1, False) is first
+    first = cache.training(w, a, 1, False)
+    assert cache.training(w, a, 1, False) is first
     a.mul_(0.5)
-    second = cache.get(w, a, 1, False)
-    assert second is not first and float(second.act_scale) == 1.5
+    second = cache.training(w, a, 1, False)
+    assert second is not first and float(second.act_scale) == 1.5 and float(first.act_scale) == 3.0
     other = w.clone()
-    assert cache.get(other, a, 1, False) is not second     # another object, equal values
+    assert cache.training(other, a, 1, False) is not second     # another object, equal values
     errors = []
 
     def passes(scale):
         try:
             mine = torch.tensor([scale], dtype=torch.bfloat16)
             for i in range(300):
-                got = cache.get(mine if i % 3 else other, a, i % 11, False)
+                got = cache.training(mine if i % 3 else other, a, i % 11, False)
                 if float(got.weight_scale) != (scale if i % 3 else 3.0):
                     errors.append(i)
         except Exception as e:                              # noqa: BLE001
@@ -140,9 +163,8 @@ def test_layers_saved_without_constants_load():
         layer.weight_global_scale.fill_(3)
         layer.act_global_scale.fill_(3)
     want = float(layer._gemm_alpha())
-    layer._constants.get(layer.weight_global_scale, layer.act_global_scale, 0, True)
     twin = copy.deepcopy(layer)
-    assert float(twin._gemm_alpha()) == want and not twin._constants._captured
+    assert not twin._constants._inference and float(twin._gemm_alpha()) == want
     del layer._constants
     loaded = pickle.loads(pickle.dumps(layer))
     assert float(loaded._gemm_alpha()) == want
