@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.cuda import is_current_stream_capturing
 
 from ... import ops
 from ...rotation import classify_rotation, sylvester
@@ -134,7 +135,7 @@ class FPQuantLinear(nn.Module):
         w, a = self.weight_global_scale, self.act_global_scale
         if not w.is_cuda:
             return self._constants.inference(w, a, 0, lambda: False)
-        return self._constants.inference(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing)
+        return self._constants.inference(w, a, ops._stream(w), is_current_stream_capturing)
 
     def _gemm_alpha(self) -> torch.Tensor:
         """1 / (weight_global_scale * act_global_scale) as fp32 [1]."""
@@ -205,7 +206,7 @@ class FPQuantLinear(nn.Module):
         w, a = self.weight_global_scale, self.act_global_scale
         if not w.is_cuda:
             return self._constants.training(w, a, 0, False)
-        return self._constants.training(w, a, ops._stream(w), torch.cuda.is_current_stream_capturing())
+        return self._constants.training(w, a, ops._stream(w), is_current_stream_capturing())
 
     # ------------------------------------------------------------------ forward
     def forward(self, x) -> torch.Tensor:

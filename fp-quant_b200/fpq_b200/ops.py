@@ -23,13 +23,14 @@ try:        # private names of torch: where one is missing, the calls below take
     _CAN_TELL = True
 except (ImportError, AttributeError):
     _CAN_TELL = False
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+_is_compiling = torch.compiler.is_compiling
 
 
 def plain_eager(x: torch.Tensor) -> bool:
     """No tracer, dispatch or function mode (but the one that sets a default device), functorch transform, forward-mode
     derivative or tensor subclass between the caller and the kernels: native calls may be made on x's address."""
-    return (_CAN_TELL and type(x) in (torch.Tensor, torch.nn.Parameter) and not torch.compiler.is_compiling()
+    return (_CAN_TELL and type(x) in _PLAIN and not _is_compiling()
             and _len_torch_dispatch_stack() == 0 and peek_interpreter_stack() is None and forward_ad._current_level < 0
             and (_len_torch_function_stack() == 0
                  or all(type(m) is DeviceContext for m in _get_current_function_mode_stack())))
@@ -49,10 +50,13 @@ def _cuda(t: torch.Tensor, name: str = "tensor") -> torch.Tensor:
     return t
 
 
-def _stream(t: torch.Tensor) -> int:
-    if _raw_stream is None:
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+if _raw_stream is not None:
+    def _stream(t: torch.Tensor) -> int:
+        return _raw_stream(t.device.index)     # without building a Stream object (1 us of 1.2)
+else:
+    def _stream(t: torch.Tensor) -> int:
         return torch.cuda.current_stream(t.device).cuda_stream
-    return _raw_stream(t.device.index)     # without building a Stream object (1 us of 1.2)
 
 
 class _NoGuard:

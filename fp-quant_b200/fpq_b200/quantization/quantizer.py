@@ -124,7 +124,7 @@ class Quantizer:
         # one kernel where it can be called on addresses, the same product in torch under a tracer, mode or transform
         if self.group_size and q.is_cuda and s.device == q.device and q.dtype in (torch.float32, torch.bfloat16) \
                 and q.dim() > 0 and s.shape == q.shape[:-1] + (q.shape[-1] // self.group_size,) \
-                and q.shape[-1] % self.group_size == 0 and ops.plain_eager(q) and ops.plain_eager(s) \
+                and q.shape[-1] % self.group_size == 0 and ops.plain_eager(q) and type(s) is torch.Tensor \
                 and q.is_contiguous() and s.is_contiguous() and q.data_ptr() % 16 == 0 and q.numel() > 0:
             return ops.multiply_scales(q, s, self.group_size)
         if self.group_size:
