@@ -118,7 +118,8 @@ __global__ void reflect_inplace_kernel(float* A, int64_t d) {
 //   phase 2   four warps, one vector a thread: the rows of C below D_p and the columns of X_p (from S_p, and from the
 //             unit vectors), by forward substitution
 //   phase 3   all: the trailing part -= C (C / pivot)^T
-// with C the unscaled columns of L and X = L^-1 by blocks of rows.
+// with C the unscaled columns of L and X = L^-1 by blocks of rows.  40 us in the chain of d = 4096; 48 us as one elimination
+// with a barrier per column; 33 us with approximate reciprocals and sums in two halves, which changed the bits.
 constexpr int CD_LD = NB + 4;         // row stride in shared memory: 16-byte rows whose starts walk through the banks
 constexpr int CD_B = 32;              // block of columns
 constexpr int CD_SLD = 96 + 4;
@@ -342,8 +343,8 @@ __global__ void __launch_bounds__(256, 1) chol_diag_kernel(float* A, int64_t lda
 // ------------------------------------------------------------------ panel below a diagonal block
 // A[i, 0..127] <- sum_k A[i, k] Linv[j, k] (k <= j, in order) in place for `rows` rows: L21 = A21 L11^-T.  A CTA takes 32 rows, so
 // that even a short panel spreads over the SMs, and holds Linv in shared memory; a thread has 2 x 8 outputs, the part
-// of Linv above its diagonal is skipped.  Latency-bound; as a 128 x 128-tile matrix product on at most 112 CTAs it took
-// 18 to 20 us a panel on average, here 10 (d = 4096) to 15 (d = 14336).
+// of Linv above its diagonal is skipped.  Latency-bound.  Panels of a chain, average under ncu: 15 us at d = 4096 and
+// 21 us at d = 14336; as a 128 x 128-tile matrix product on at most 112 CTAs 21 and 20 us.
 constexpr int PANEL_ROWS = 32;
 constexpr int PANEL_SMEM = (NB + PANEL_ROWS) * CD_LD * (int)sizeof(float);
 
