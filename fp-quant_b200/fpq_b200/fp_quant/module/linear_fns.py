@@ -59,7 +59,7 @@ class ConstantsCache:
     training step otherwise).  The tensors a set was made from are kept and compared as objects, so an address that is used
     again cannot pass for them.  One set per stream, so that no stream reads what another one may not have written yet.
     Nothing made while the stream is being captured is kept: its values only exist after a replay."""
-    STREAMS = 8
+    STREAMS = 64        # torch hands out 32 streams a priority in turn; a set is three blocks of 512 bytes
 
     def __init__(self):
         self._training = None       # (scales, {stream: set}), replaced as a whole: threads see one state or the other
